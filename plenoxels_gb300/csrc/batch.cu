@@ -100,23 +100,20 @@ __device__ __forceinline__ uint32_t cell_occupied(const pgb_scene& sc, uint64_t 
 
 // Clears the gradient-pass bits of a sample's corners that are not occupied (unoccupied
 // cells are not parameters), in the bit layout of sample_value.
-template <int MODE>
+template <int MODE, int A>
 __device__ __forceinline__ uint32_t occupied_bits(const pgb_scene& sc, const GridP<float>& g,
                                                   float nx, float ny, float nz, uint32_t bits) {
   if (sc.occupancy == nullptr || bits == 0u) return bits;
   if (MODE == PGB_NEAREST) {
-    const uint64_t c = cell_index(g, (int)rintf(nx), (int)rintf(ny), (int)rintf(nz));
-    return cell_occupied(sc, c) ? bits : 0u;
+    uint64_t c;
+    return nearest_cell<A>(g, nx, ny, nz, c) && cell_occupied(sc, c) ? bits : 0u;
   }
   Corners<float> q;
-  trilinear_corners(g, nx, ny, nz, q);
+  trilinear_corners<A>(g, nx, ny, nz, q);
+  const CornerCells<A, float> cells(g, q);
 #pragma unroll
-  for (int corner = 0; corner < 8; ++corner) {
-    const int ix = (corner & 4) ? q.f[0] : q.c[0];
-    const int iy = (corner & 2) ? q.f[1] : q.c[1];
-    const int iz = (corner & 1) ? q.f[2] : q.c[2];
-    if (!cell_occupied(sc, cell_index(g, ix, iy, iz))) bits &= ~(0xfu << (4 * corner));
-  }
+  for (int corner = 0; corner < 8; ++corner)
+    if (!cell_occupied(sc, cells(corner))) bits &= ~(0xfu << (4 * corner));
   return bits;
 }
 
@@ -128,17 +125,17 @@ __device__ __forceinline__ uint32_t occupied_bits(const pgb_scene& sc, const Gri
 
 // One sample of a batched ray: coordinates, the brick test and, unless skipped, the value
 // and its gradient-pass bits (occupancy folded in). Returns whether it was looked up.
-template <typename Store, int MODE>
+template <typename Store, int MODE, int A>
 PGB_BATCH_GATHER_ATTR bool batch_sample(const RenderArgs<float>& ra, const Ray<float>& ray,
-                                        const pgb_scene& sc, int s, float v[4], uint32_t& bits,
-                                        float& nx, float& ny, float& nz) {
+                                        const pgb_scene& sc, int s, int end, float v[4],
+                                        uint32_t& bits, float& nx, float& ny, float& nz) {
   v[0] = v[1] = v[2] = v[3] = 0.f;
   bits = 0u;
-  if (s >= ra.S) return false;
-  sample_coords(ra, ray, s, nx, ny, nz);
+  if (s >= end) return false;
+  sample_coords<A>(ra, ray, s, nx, ny, nz);
   if (brick_clear(sc, nx, ny, nz)) return false;
-  sample_value<float, Store, MODE>(ra.g, nx, ny, nz, v, bits);
-  bits = occupied_bits<MODE>(sc, ra.g, nx, ny, nz, bits);
+  sample_value<float, Store, MODE, A, true>(ra.g, nx, ny, nz, v, bits);
+  bits = occupied_bits<MODE, A>(sc, ra.g, nx, ny, nz, bits);
   return true;
 }
 
@@ -155,11 +152,203 @@ template <int K>
 using BatchStage = ChunkStage<float, K, (K == 1 ? PGB_BATCH_STAGE_CHUNKS : 1),
                               (K != 1 || PGB_BATCH_STAGE_COORDS != 0)>;
 
-// MERGE: the trilinear scatter merges the warp's updates of the same cell
-// (warp_merged_scatter) before its atomics.
+// Bytes of one warp's scene arguments in shared memory (the stage behind them stays aligned).
+constexpr int kSceneArgsBytes = ((int)sizeof(RenderArgs<float>) + 15) & ~15;
+
+// A scene as the single-scene kernels see it.
+__device__ __forceinline__ void scene_args(const BatchArgs& a, const pgb_scene& sc,
+                                           RenderArgs<float>& ra) {
+  ra.g.cells = sc.cells;
+  ra.g.X = sc.dims[0]; ra.g.Y = sc.dims[1]; ra.g.Z = sc.dims[2];
+  ra.g.fX = (float)sc.dims[0]; ra.g.fY = (float)sc.dims[1]; ra.g.fZ = (float)sc.dims[2];
+  ra.g.ox = sc.origin[0]; ra.g.oy = sc.origin[1]; ra.g.oz = sc.origin[2];
+  ra.g.pd = sc.points_distance;
+  ra.g.inv_pd = 1.0f / sc.points_distance;
+  ra.g.quick = quick_grid(sc.dims[0], sc.dims[1], sc.dims[2], sc.origin[0], sc.origin[1],
+                          sc.origin[2], sc.points_distance) ? 1 : 0;
+  ra.g.clip = a.clip;
+  ra.g.alpha_floor = 0.f;
+  ra.S = sc.num_samples;
+  ra.delta = sc.delta_step;
+  ra.stratified = a.stratified;
+  ra.grad = reinterpret_cast<float*>(sc.grad_cells);
+}
+
+// One ray of the batch: sampling, lookup, compositing, squared error and adjoint on its own
+// scene. MERGE: the trilinear scatter merges the warp's updates of the same cell
+// (warp_merged_scatter) before its atomics. A: the index arithmetic (Arith).
+template <typename Store, int MODE, int K, bool MERGE, int A>
+__device__ __forceinline__ void batch_ray(const BatchArgs& a, const pgb_scene& sc,
+                                          const RenderArgs<float>& ra, int64_t r, BatchStage<K> cs,
+                                          int lane) {
+  const float grad_scale = a.grad_scale;  // d(weighted MSE)/d pixel
+  float* grad = ra.grad;
+  Ray<float> ray;
+  ray.ox = a.origins[3 * r + 0]; ray.oy = a.origins[3 * r + 1]; ray.oz = a.origins[3 * r + 2];
+  ray.dx = a.dirs[3 * r + 0];    ray.dy = a.dirs[3 * r + 1];    ray.dz = a.dirs[3 * r + 2];
+  ray.tgt = a.target[4 * r + (lane & 3)];
+  ray.h = a.stratified ? hash_stream(a.seed, (uint64_t)r) : 0ull;
+
+  if (ra.S > kWarp * kWarp * K) {  // a chunk start per lane: more chunks are not supported
+    if (lane == 0) a.ray_loss[r] = __int_as_float(0x7fc00000);  // NaN loss
+    if (a.rgba_out != nullptr && lane < 4) a.rgba_out[4 * r + lane] = __int_as_float(0x7fc00000);
+    return;
+  }
+  int first, end;
+  ray_span(ra, ray, first, end);
+  first -= first % (kWarp * K);  // chunks stay where they were: T is looked at after each
+  const int nchunks = (end - first + kWarp * K - 1) / (kWarp * K);
+  float v[K][4];
+  uint32_t bits[K];
+  float Ts[K];
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  float T = 1.f, Tstart = 1.f;
+  int last = -1;
+
+  auto gather = [&](int c) {
+#if PGB_BATCH_LOOP
+#pragma unroll 1
+    for (int k = 0; k < K; ++k) {
+      float t[4], nx, ny, nz;
+      uint32_t b;
+      if (batch_sample<Store, MODE, A>(ra, ray, sc, first + (c * K + k) * kWarp + lane, end, t, b, nx, ny,
+                                    nz))
+        cs.put(c, k, lane, nx, ny, nz);
+#pragma unroll
+      for (int kk = 0; kk < K; ++kk) {
+        if (kk == k) {
+          v[kk][0] = t[0]; v[kk][1] = t[1]; v[kk][2] = t[2]; v[kk][3] = t[3];
+          bits[kk] = b;
+        }
+      }
+    }
+#else
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      float nx, ny, nz;
+      if (batch_sample<Store, MODE, A>(ra, ray, sc, first + (c * K + k) * kWarp + lane, end, v[k],
+                                    bits[k], nx, ny, nz))
+        cs.put(c, k, lane, nx, ny, nz);
+    }
+#endif
+  };
+
+  for (int c = 0; c < nchunks; ++c) {
+    if (lane == c) Tstart = T;
+    __syncwarp();
+    gather(c);
+#pragma unroll
+    for (int k = 0; k < K; ++k) cs.put_vals(c, k, lane, v[k], bits[k]);
+    T = scan_chunk<float, K>(v, T, lane, Ts);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const float w = v[k][3] * Ts[k];
+      acc[0] += w * v[k][0];
+      acc[1] += w * v[k][1];
+      acc[2] += w * v[k][2];
+      acc[3] += w;
+    }
+    last = c;
+    if (a.term_thr > 0.0f && T < a.term_thr) break;
+  }
+  float px[4];
+#pragma unroll
+  for (int ch = 0; ch < 4; ++ch) px[ch] = warp_sum(acc[ch]);
+  float gpx[4];
+  float sq = 0.f;
+#pragma unroll
+  for (int ch = 0; ch < 4; ++ch) {
+    const float diff = px[ch] - __shfl_sync(kFull, ray.tgt, ch);
+    sq += diff * diff;
+    gpx[ch] = grad_scale * diff;
+  }
+  if (lane == 0) a.ray_loss[r] = sq;
+  if (a.rgba_out != nullptr && lane < 4) a.rgba_out[4 * r + lane] = pick4(px, lane);
+
+  float Snext_carry = 0.f;
+  for (int c = last; c >= 0; --c) {
+    if (c != last) {
+      __syncwarp();
+      if (BatchStage<K>::holds(c, last)) {  // the chunk's values are still staged
+#pragma unroll
+        for (int k = 0; k < K; ++k) cs.get_vals(c, k, lane, v[k], bits[k]);
+      } else {
+        gather(c);
+      }
+      scan_chunk<float, K>(v, __shfl_sync(kFull, Tstart, c), lane, Ts);
+    }
+    __syncwarp();
+#if PGB_BATCH_LOOP
+#pragma unroll 1
+#else
+#pragma unroll
+#endif
+    for (int k = K - 1; k >= 0; --k) {
+      float vk[4], tk;
+      uint32_t bk;
+#pragma unroll
+      for (int kk = 0; kk < K; ++kk) {
+        if (kk == k) {
+          vk[0] = v[kk][0]; vk[1] = v[kk][1]; vk[2] = v[kk][2]; vk[3] = v[kk][3];
+          bk = bits[kk];
+          tk = Ts[kk];
+        }
+      }
+      // a slot with alpha 0 and nothing to scatter leaves S unchanged (identity maps)
+      if (PGB_SLOT_SKIP && !__any_sync(kFull, bk != 0u || vk[3] != 0.f)) continue;
+      const float al = vk[3];
+      const float G = gpx[0] * vk[0] + gpx[1] * vk[1] + gpx[2] * vk[2] + gpx[3];
+      float fa = G * al, fb = 1.f - al;
+      warp_suffix_affine(fa, fb, lane);
+      const float S_here = fa + fb * Snext_carry;
+      float S_after = __shfl_down_sync(kFull, S_here, 1);
+      if (lane == kWarp - 1) S_after = Snext_carry;
+      Snext_carry = __shfl_sync(kFull, S_here, 0);
+      if (MERGE && MODE == PGB_TRILINEAR) {
+        float dv[4] = {0.f, 0.f, 0.f, 0.f};
+        float nx = 0.f, ny = 0.f, nz = 0.f;
+        bool has = false;
+        if (bk != 0u) {
+          const float w = al * tk;
+          dv[0] = gpx[0] * w; dv[1] = gpx[1] * w; dv[2] = gpx[2] * w;
+          dv[3] = tk * (G - S_after);
+          has = dv[0] != 0.f || dv[1] != 0.f || dv[2] != 0.f || dv[3] != 0.f;
+          if (has) {
+            if constexpr (BatchStage<K>::kHasCoords)
+              cs.get(c, k, lane, nx, ny, nz);
+            else
+              sample_coords<A>(ra, ray, first + (c * K + k) * kWarp + lane, nx, ny, nz);
+          }
+        }
+        warp_merged_scatter<float, A>(ra.g, grad, has, nx, ny, nz, dv, bk, lane);
+      } else if (bk != 0u) {
+        const float w = al * tk;
+        float dv[4] = {gpx[0] * w, gpx[1] * w, gpx[2] * w, tk * (G - S_after)};
+        if (!(dv[0] != 0.f || dv[1] != 0.f || dv[2] != 0.f || dv[3] != 0.f)) continue;
+        float nx, ny, nz;
+        if constexpr (BatchStage<K>::kHasCoords)
+          cs.get(c, k, lane, nx, ny, nz);
+        else
+          sample_coords<A>(ra, ray, first + (c * K + k) * kWarp + lane, nx, ny, nz);
+        sample_scatter<float, MODE, A>(ra.g, grad, nx, ny, nz, dv, bk);
+      }
+    }
+  }
+}
+
+// Scenes outside the quick index arithmetic's range go through a call of their own, so
+// that the kernel's registers are those of the quick form (with both forms inline, its 80
+// registers spilled 264 bytes).
+template <typename Store, int MODE, int K, bool MERGE>
+__device__ __noinline__ void batch_ray_general(const BatchArgs& a, const pgb_scene& sc,
+                                               const RenderArgs<float>& ra, int64_t r,
+                                               BatchStage<K> cs, int lane) {
+  batch_ray<Store, MODE, K, MERGE, kGeneral>(a, sc, ra, r, cs, lane);
+}
+
 template <typename Store, int MODE, int K, bool MERGE>
 __global__ void __launch_bounds__(kBatchMaxThreads, K == 1 ? PGB_BATCH_MIN_BLOCKS_K1 : PGB_BATCH_MIN_BLOCKS)
-    batch_train_kernel(const BatchArgs a) {
+    batch_train_kernel(const __grid_constant__ BatchArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pgb_scene* sc_tab = reinterpret_cast<pgb_scene*>(smem_raw);
   const size_t tab_bytes = ((size_t)a.num_scenes * sizeof(pgb_scene) + 15) & ~(size_t)15;
@@ -172,8 +361,13 @@ __global__ void __launch_bounds__(kBatchMaxThreads, K == 1 ? PGB_BATCH_MIN_BLOCK
   __syncthreads();
   const int lane = threadIdx.x & (kWarp - 1);
   const int wib = threadIdx.x >> 5;
-  BatchStage<K> cs(smem_raw + tab_bytes, wib);
-  const float grad_scale = a.grad_scale;  // d(weighted MSE)/d pixel
+  // The arguments of the scene that the warp's ray belongs to, one copy per warp, rewritten
+  // when a ray of another scene comes (they are read where they are used: as local variables
+  // they and their spills took 140 bytes of stack in the 80-register kernel).
+  RenderArgs<float>& ra =
+      *reinterpret_cast<RenderArgs<float>*>(smem_raw + tab_bytes + (size_t)wib * kSceneArgsBytes);
+  int current = -1;
+  BatchStage<K> cs(smem_raw + tab_bytes + (size_t)kSceneArgsBytes * (blockDim.x / kWarp), wib);
 
   for (;;) {
     unsigned long long rr = 0;
@@ -189,167 +383,16 @@ __global__ void __launch_bounds__(kBatchMaxThreads, K == 1 ? PGB_BATCH_MIN_BLOCK
     }
     const pgb_scene& sc = sc_tab[sid];
 
-    // the ray's scene as the single-scene kernels see it
-    RenderArgs<float> ra = {};
-    ra.g.cells = sc.cells;
-    ra.g.X = sc.dims[0]; ra.g.Y = sc.dims[1]; ra.g.Z = sc.dims[2];
-    ra.g.fX = (float)ra.g.X; ra.g.fY = (float)ra.g.Y; ra.g.fZ = (float)ra.g.Z;
-    ra.g.ox = sc.origin[0]; ra.g.oy = sc.origin[1]; ra.g.oz = sc.origin[2];
-    ra.g.pd = sc.points_distance;
-    ra.g.clip = a.clip;
-    ra.S = sc.num_samples;
-    ra.delta = sc.delta_step;
-    ra.stratified = a.stratified;
-    ra.strat_seed = a.seed;
-    float* grad = reinterpret_cast<float*>(sc.grad_cells);
-
-    Ray<float> ray;
-    ray.ox = a.origins[3 * r + 0]; ray.oy = a.origins[3 * r + 1]; ray.oz = a.origins[3 * r + 2];
-    ray.dx = a.dirs[3 * r + 0];    ray.dy = a.dirs[3 * r + 1];    ray.dz = a.dirs[3 * r + 2];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) ray.tgt[c] = a.target[4 * r + c];
-    ray.h = a.stratified ? hash_stream(a.seed, (uint64_t)r) : 0ull;
-
-    const int nchunks = (ra.S + kWarp * K - 1) / (kWarp * K);
-    if (nchunks > kWarp) {  // a chunk start per lane: more chunks are not supported
-      if (lane == 0) a.ray_loss[r] = __int_as_float(0x7fc00000);  // NaN loss
-      if (a.rgba_out != nullptr && lane < 4) a.rgba_out[4 * r + lane] = __int_as_float(0x7fc00000);
-      continue;
-    }
-    float v[K][4];
-    uint32_t bits[K];
-    float Ts[K];
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    float T = 1.f, Tstart = 1.f;
-    int last = -1;
-
-    auto gather = [&](int c) {
-#if PGB_BATCH_LOOP
-#pragma unroll 1
-      for (int k = 0; k < K; ++k) {
-        float t[4], nx, ny, nz;
-        uint32_t b;
-        if (batch_sample<Store, MODE>(ra, ray, sc, (c * K + k) * kWarp + lane, t, b, nx, ny, nz))
-          cs.put(c, k, lane, nx, ny, nz);
-#pragma unroll
-        for (int kk = 0; kk < K; ++kk) {
-          if (kk == k) {
-            v[kk][0] = t[0]; v[kk][1] = t[1]; v[kk][2] = t[2]; v[kk][3] = t[3];
-            bits[kk] = b;
-          }
-        }
-      }
-#else
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        float nx, ny, nz;
-        if (batch_sample<Store, MODE>(ra, ray, sc, (c * K + k) * kWarp + lane, v[k], bits[k], nx, ny, nz))
-          cs.put(c, k, lane, nx, ny, nz);
-      }
-#endif
-    };
-
-    for (int c = 0; c < nchunks; ++c) {
-      if (lane == c) Tstart = T;
+    if (sid != current) {
       __syncwarp();
-      gather(c);
-#pragma unroll
-      for (int k = 0; k < K; ++k) cs.put_vals(c, k, lane, v[k], bits[k]);
-      T = scan_chunk<float, K>(v, T, lane, Ts);
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const float w = v[k][3] * Ts[k];
-        acc[0] += w * v[k][0];
-        acc[1] += w * v[k][1];
-        acc[2] += w * v[k][2];
-        acc[3] += w;
-      }
-      last = c;
-      if (a.term_thr > 0.0f && T < a.term_thr) break;
-    }
-    float px[4];
-#pragma unroll
-    for (int ch = 0; ch < 4; ++ch) px[ch] = warp_sum(acc[ch]);
-    float gpx[4];
-    float sq = 0.f;
-#pragma unroll
-    for (int ch = 0; ch < 4; ++ch) {
-      const float diff = px[ch] - ray.tgt[ch];
-      sq += diff * diff;
-      gpx[ch] = grad_scale * diff;
-    }
-    if (lane == 0) a.ray_loss[r] = sq;
-    if (a.rgba_out != nullptr && lane < 4) a.rgba_out[4 * r + lane] = pick4(px, lane);
-
-    float Snext_carry = 0.f;
-    for (int c = last; c >= 0; --c) {
-      if (c != last) {
-        __syncwarp();
-        if (BatchStage<K>::holds(c, last)) {  // the chunk's values are still staged
-#pragma unroll
-          for (int k = 0; k < K; ++k) cs.get_vals(c, k, lane, v[k], bits[k]);
-        } else {
-          gather(c);
-        }
-        scan_chunk<float, K>(v, __shfl_sync(kFull, Tstart, c), lane, Ts);
-      }
+      if (lane == 0) scene_args(a, sc, ra);
       __syncwarp();
-#if PGB_BATCH_LOOP
-#pragma unroll 1
-#else
-#pragma unroll
-#endif
-      for (int k = K - 1; k >= 0; --k) {
-        float vk[4], tk;
-        uint32_t bk;
-#pragma unroll
-        for (int kk = 0; kk < K; ++kk) {
-          if (kk == k) {
-            vk[0] = v[kk][0]; vk[1] = v[kk][1]; vk[2] = v[kk][2]; vk[3] = v[kk][3];
-            bk = bits[kk];
-            tk = Ts[kk];
-          }
-        }
-        // a slot with alpha 0 and nothing to scatter leaves S unchanged (identity maps)
-        if (PGB_SLOT_SKIP && !__any_sync(kFull, bk != 0u || vk[3] != 0.f)) continue;
-        const float al = vk[3];
-        const float G = gpx[0] * vk[0] + gpx[1] * vk[1] + gpx[2] * vk[2] + gpx[3];
-        float fa = G * al, fb = 1.f - al;
-        warp_suffix_affine(fa, fb, lane);
-        const float S_here = fa + fb * Snext_carry;
-        float S_after = __shfl_down_sync(kFull, S_here, 1);
-        if (lane == kWarp - 1) S_after = Snext_carry;
-        Snext_carry = __shfl_sync(kFull, S_here, 0);
-        if (MERGE && MODE == PGB_TRILINEAR) {
-          float dv[4] = {0.f, 0.f, 0.f, 0.f};
-          float nx = 0.f, ny = 0.f, nz = 0.f;
-          bool has = false;
-          if (bk != 0u) {
-            const float w = al * tk;
-            dv[0] = gpx[0] * w; dv[1] = gpx[1] * w; dv[2] = gpx[2] * w;
-            dv[3] = tk * (G - S_after);
-            has = dv[0] != 0.f || dv[1] != 0.f || dv[2] != 0.f || dv[3] != 0.f;
-            if (has) {
-              if constexpr (BatchStage<K>::kHasCoords)
-                cs.get(c, k, lane, nx, ny, nz);
-              else
-                sample_coords(ra, ray, (c * K + k) * kWarp + lane, nx, ny, nz);
-            }
-          }
-          warp_merged_scatter<float>(ra.g, grad, has, nx, ny, nz, dv, bk, lane);
-        } else if (bk != 0u) {
-          const float w = al * tk;
-          float dv[4] = {gpx[0] * w, gpx[1] * w, gpx[2] * w, tk * (G - S_after)};
-          if (!(dv[0] != 0.f || dv[1] != 0.f || dv[2] != 0.f || dv[3] != 0.f)) continue;
-          float nx, ny, nz;
-          if constexpr (BatchStage<K>::kHasCoords)
-            cs.get(c, k, lane, nx, ny, nz);
-          else
-            sample_coords(ra, ray, (c * K + k) * kWarp + lane, nx, ny, nz);
-          sample_scatter<float, MODE>(ra.g, grad, nx, ny, nz, dv, bk);
-        }
-      }
+      current = sid;
     }
+    if (ra.g.quick)
+      batch_ray<Store, MODE, K, MERGE, kQuick>(a, sc, ra, r, cs, lane);
+    else
+      batch_ray_general<Store, MODE, K, MERGE>(a, sc, ra, r, cs, lane);
   }
 
   // the last block to finish resets the queue (ray_loss_sum_kernel, launched next, sums
@@ -489,13 +532,13 @@ template <typename Store, int MODE, int K, bool MERGE>
 int launch_batch_k(const BatchArgs& a, int threads, cudaStream_t s) {
   const int warps = threads / kWarp;
   const size_t tab = (((size_t)a.num_scenes * sizeof(pgb_scene)) + 15) & ~(size_t)15;
-  const size_t smem = tab + (size_t)BatchStage<K>::kBytesPerWarp * warps;
+  const size_t smem = tab + (kSceneArgsBytes + (size_t)BatchStage<K>::kBytesPerWarp) * warps;
   auto kern = batch_train_kernel<Store, MODE, K, MERGE>;
   int dev = 0;
   cudaGetDevice(&dev);
   static int configured[64] = {0};
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) != cudaSuccess)
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024) != cudaSuccess)
       return PGB_ERR_LAUNCH;
     configured[dev] = 1;
   }

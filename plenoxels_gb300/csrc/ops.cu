@@ -535,7 +535,7 @@ __global__ void render_indices_kernel(const RenderArgs<Real> a, int64_t* __restr
     Ray<Real> ray;
     load_ray(a, r, ray, false);
     Real nx, ny, nz;
-    sample_coords(a, ray, s, nx, ny, nz);
+    sample_coords<kByGrid>(a, ray, s, nx, ny, nz);
     if (MODE == PGB_NEAREST) {
       long long idx[3];
       bool inb;
@@ -789,7 +789,7 @@ __global__ void render_coords_kernel(const RenderArgs<Real> a, Real* __restrict_
     Ray<Real> ray;
     load_ray(a, r, ray, false);
     Real nx, ny, nz;
-    sample_coords(a, ray, s, nx, ny, nz);
+    sample_coords<kByGrid>(a, ray, s, nx, ny, nz);
     out[3 * i + 0] = nx;
     out[3 * i + 1] = ny;
     out[3 * i + 2] = nz;

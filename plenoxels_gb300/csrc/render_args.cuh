@@ -4,6 +4,8 @@
 // same kernels.
 #pragma once
 
+#include <cmath>
+
 #include "pgb_host.h"
 #include "render.cuh"
 
@@ -31,6 +33,9 @@ GridP<Real> grid_params(const pgb_grid* g) {
   p.fX = (Real)p.X; p.fY = (Real)p.Y; p.fZ = (Real)p.Z;
   p.ox = (Real)g->origin[0]; p.oy = (Real)g->origin[1]; p.oz = (Real)g->origin[2];
   p.pd = (Real)g->points_distance;
+  p.inv_pd = Real(1) / p.pd;
+  p.quick = sizeof(Real) == 4 && quick_grid(p.X, p.Y, p.Z, (float)p.ox, (float)p.oy, (float)p.oz,
+                                            (float)p.pd) ? 1 : 0;
   p.clip = g->clip ? 1 : 0;
   p.alpha_floor = g->alpha_floor;
   return p;
@@ -97,6 +102,7 @@ void finish_args(RenderArgs<Real>& a) {
   a.grad_scale = (Real)(2.0 * a.loss_w * a.inv_count);
   // beta_w / (R*S) * (1 + 2 eps): the numerator of 1/(alpha+eps) + 1/(1-alpha+eps)
   a.beta_scale = (Real)(a.beta_w * a.inv_samples * (1.0 + 2.0 * (double)a.beta_eps));
+  a.beta_zero = (Real)(std::log((double)a.beta_eps) - std::log(1.0 + (double)a.beta_eps));
 }
 
 template <typename Real>

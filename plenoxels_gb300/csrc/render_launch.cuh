@@ -11,7 +11,7 @@
 
 namespace pgb {
 
-template <typename Real, typename Store, int MODE, int K, int PHASE, bool LOGT>
+template <typename Real, typename Store, int MODE, int K, int PHASE, bool LOGT, int A>
 int launch_render_k(const RenderArgs<Real>& a, cudaStream_t s) {
   constexpr int kThreads = render_threads<MODE, K>();
   constexpr int kWarpsPerBlock = kThreads / kWarp;
@@ -22,7 +22,7 @@ int launch_render_k(const RenderArgs<Real>& a, cudaStream_t s) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    if (cudaFuncSetAttribute(render_kernel<Real, Store, MODE, K, PHASE, LOGT>,
+    if (cudaFuncSetAttribute(render_kernel<Real, Store, MODE, K, PHASE, LOGT, A>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess)
       return PGB_ERR_LAUNCH;
     configured[dev] = 1;
@@ -31,19 +31,26 @@ int launch_render_k(const RenderArgs<Real>& a, cudaStream_t s) {
   blocks = std::min<int64_t>(blocks, PHASE == kTrain ? kMaxTrainWarps / kWarpsPerBlock
                                                      : (int64_t)1 << 20);
   if (blocks < 1) blocks = 1;
-  render_kernel<Real, Store, MODE, K, PHASE, LOGT><<<(unsigned)blocks, kThreads, kSmem, s>>>(a);
+  render_kernel<Real, Store, MODE, K, PHASE, LOGT, A><<<(unsigned)blocks, kThreads, kSmem, s>>>(a);
   return after_launch();
 }
 
 template <typename Real, typename Store, int MODE, int PHASE, bool LOGT>
 int launch_render_mp(const RenderArgs<Real>& a, cudaStream_t s) {
+  // Grids outside the quick index arithmetic's range (a dimension of one cell or above
+  // 2^21, 2^32 cells): one kernel with the general arithmetic serves every ray length.
+  // fp64 grids have the general arithmetic throughout.
+  constexpr int A = sizeof(Real) == 4 ? kQuick : kGeneral;
+  if constexpr (A == kQuick) {
+    if (!a.g.quick) return launch_render_k<Real, Store, MODE, 8, PHASE, LOGT, kGeneral>(a, s);
+  }
   const bool early_stop = a.g.clip && !(PHASE == kTrain && a.beta_w != 0.0);
   switch (pick_slots(a.S, a.chunk_samples, early_stop, MODE)) {
-    case 1: return launch_render_k<Real, Store, MODE, 1, PHASE, LOGT>(a, s);
-    case 2: return launch_render_k<Real, Store, MODE, 2, PHASE, LOGT>(a, s);
-    case 4: return launch_render_k<Real, Store, MODE, 4, PHASE, LOGT>(a, s);
-    case 8: return launch_render_k<Real, Store, MODE, 8, PHASE, LOGT>(a, s);
-    case 16: return launch_render_k<Real, Store, MODE, 16, PHASE, LOGT>(a, s);
+    case 1: return launch_render_k<Real, Store, MODE, 1, PHASE, LOGT, A>(a, s);
+    case 2: return launch_render_k<Real, Store, MODE, 2, PHASE, LOGT, A>(a, s);
+    case 4: return launch_render_k<Real, Store, MODE, 4, PHASE, LOGT, A>(a, s);
+    case 8: return launch_render_k<Real, Store, MODE, 8, PHASE, LOGT, A>(a, s);
+    case 16: return launch_render_k<Real, Store, MODE, 16, PHASE, LOGT, A>(a, s);
     default: return PGB_ERR_UNSUPPORTED;
   }
 }
