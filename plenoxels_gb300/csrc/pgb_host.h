@@ -43,31 +43,35 @@ int launch_render_f64(const RenderArgs<double>& a, int mode, int phase, cudaStre
 int launch_render_logt_f32(const RenderArgs<float>& a, int mode, int phase, cudaStream_t s);
 int launch_render_logt_bf16(const RenderArgs<float>& a, int mode, int phase, cudaStream_t s);
 
-// Slots per lane (K) of a chunk of 32 * K samples. A requested chunk size (32 * K for K
-// in 1, 2, 4, 8, 16) is raised until a ray spans at most kMaxChunks chunks. Without one:
-// when rays can stop at the first chunk whose transmittance reaches 0 (clip on, no beta
-// term), short chunks (32 samples for trilinear lookup, 64 for nearest) skip the most
-// samples behind opaque cells (measured on GB300: 256^3 grid, 8192 rays x 256 samples,
-// trilinear step 0.175 ms with one 256-sample chunk, 0.133 ms with 32-sample chunks);
-// otherwise a ray up to 512 samples is a single chunk and longer rays use 256-sample
-// chunks.
-inline int pick_slots(int S, int chunk_samples = 0, bool early_stop = false,
-                      int mode = PGB_TRILINEAR) {
+// Slots per lane (K) of a chunk of 32 * K samples. A chunk size (32 * K for K in 1, 2, 4, 8,
+// 16) is raised until a ray spans at most kMaxChunks chunks. Without a requested one: 32
+// samples for trilinear lookup, 64 for nearest. Short chunks skip the most samples behind
+// opaque cells where a ray may stop there, and hold fewer registers where it may not (the
+// beta term, no clip). Measured on GB300, one training launch, chunks of 32 / 64 / 128 / 256
+// samples: 256^3 trilinear, 8192 rays x 256 with early stop 80 / 96 / 105 / 162 us; 7500
+// rays x 600 with the beta term trilinear 359 / 380 / 403 / 569 us, nearest 146 / 132 / 134
+// / 189 us (256 was the choice there before); nearest without it 105 / 92 / 92 / 127 us.
+// `long_chunks` (long_chunks_for) keeps whole rays up to 512 samples in one chunk.
+inline int pick_slots(int S, int chunk_samples = 0, int mode = PGB_TRILINEAR,
+                      bool long_chunks = false) {
 #ifdef PGB_FORCE_SLOTS
   if (S <= 32 * kMaxChunks * PGB_FORCE_SLOTS) return PGB_FORCE_SLOTS;
 #endif
-  if (chunk_samples <= 0 && early_stop) chunk_samples = mode == PGB_NEAREST ? 64 : 32;
-  if (chunk_samples > 0) {
-    int k = 1;
-    while (k < 16 && 32 * k < chunk_samples) k *= 2;
-    while (k < 16 && (S + 32 * k - 1) / (32 * k) > kMaxChunks) k *= 2;
-    return k;
-  }
-  if (S <= 64) return 2;
-  if (S <= 128) return 4;
-  if (S <= 256) return 8;
-  if (S <= 512) return 16;
-  return 8;
+  if (chunk_samples <= 0 && long_chunks) return S <= 64 ? 2 : S <= 128 ? 4 : S <= 256 || S > 512 ? 8 : 16;
+  if (chunk_samples <= 0) chunk_samples = mode == PGB_NEAREST ? 64 : 32;
+  int k = 1;
+  while (k < 16 && 32 * k < chunk_samples) k *= 2;
+  while (k < 16 && (S + 32 * k - 1) / (32 * k) > kMaxChunks) k *= 2;
+  return k;
+}
+
+// Long chunks where a ray may not stop early, (a) with a threshold on T, which is looked at
+// after each chunk, and (b) for the trilinear gradient of up to 256 samples, where there is
+// nothing to skip and one gather of the ray keeps the most loads in flight (8192 rays of 64 /
+// 128 / 256 samples, 200^3, no clip: 78 / 126 / 185 us against 85 / 139 / 190 us in chunks
+// of 32).
+inline bool long_chunks_for(int S, int mode, bool early_stop, bool gradient, float term_threshold) {
+  return !early_stop && (term_threshold > 0.f || (mode == PGB_TRILINEAR && gradient && S <= 256));
 }
 
 }  // namespace pgb

@@ -45,7 +45,8 @@ int launch_render_mp(const RenderArgs<Real>& a, cudaStream_t s) {
     if (!a.g.quick) return launch_render_k<Real, Store, MODE, 8, PHASE, LOGT, kGeneral>(a, s);
   }
   const bool early_stop = a.g.clip && !(PHASE == kTrain && a.beta_w != 0.0);
-  switch (pick_slots(a.S, a.chunk_samples, early_stop, MODE)) {
+  const bool long_chunks = long_chunks_for(a.S, MODE, early_stop, PHASE != kForward, a.term_thr);
+  switch (pick_slots(a.S, a.chunk_samples, MODE, long_chunks)) {
     case 1: return launch_render_k<Real, Store, MODE, 1, PHASE, LOGT, A>(a, s);
     case 2: return launch_render_k<Real, Store, MODE, 2, PHASE, LOGT, A>(a, s);
     case 4: return launch_render_k<Real, Store, MODE, 4, PHASE, LOGT, A>(a, s);
