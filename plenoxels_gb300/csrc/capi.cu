@@ -68,7 +68,10 @@ int render_common(const pgb_grid* g, const pgb_rays* r, int phase, void* rgba_ou
   if (workspace) {
     a.partials = (double*)workspace;
     a.partials_beta = (double*)workspace + kMaxTrainWarps;
-    a.counter = (unsigned*)((char*)workspace + 2 * sizeof(double) * kMaxTrainWarps);
+    char* behind = (char*)workspace + 2 * sizeof(double) * kMaxTrainWarps;
+    a.counter = (unsigned*)behind;
+    static_assert(sizeof(TrainState) <= kTrainStateBytes, "workspace layout");
+    a.state = (TrainState*)(behind + kTrainStateOffset);
   }
   a.loss_w = loss_w;
   a.inv_count = r->num_rays > 0 ? 1.0 / (4.0 * (double)r->num_rays) : std::nan("");
@@ -111,7 +114,7 @@ int pgb_render_bwd(const pgb_grid* grid, const pgb_rays* rays, const void* d_rgb
 }
 
 int64_t pgb_train_workspace_bytes(void) {
-  return (int64_t)2 * sizeof(double) * kMaxTrainWarps + 256;
+  return (int64_t)2 * sizeof(double) * kMaxTrainWarps + kTrainStateOffset + kTrainStateBytes;
 }
 
 int pgb_render_train(const pgb_grid* grid, const pgb_rays* rays, const void* target,

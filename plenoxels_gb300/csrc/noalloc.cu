@@ -16,17 +16,17 @@
 namespace pgb {
 namespace {
 
-// One ray per warp, so a call of at most PGB_NOALLOC_MAX_RAYS rays launches at most
-// kNoAllocMaxBlocks blocks (of the smallest render block), each writing one loss partial.
-constexpr int kNoAllocWarpsPerBlock = kRenderMinThreads / kWarp;
+// fp64 launches have one ray per warp, so a call of at most PGB_NOALLOC_MAX_RAYS rays launches
+// at most kNoAllocMaxBlocks blocks, each writing one loss partial.
+constexpr int kNoAllocWarpsPerBlock = kRenderMinThreads64 / kWarp;
 constexpr int kNoAllocMaxBlocks = PGB_NOALLOC_MAX_RAYS / kNoAllocWarpsPerBlock;
 static_assert(PGB_NOALLOC_MAX_RAYS % kNoAllocWarpsPerBlock == 0, "ray limit must fill whole blocks");
 static_assert(kNoAllocMaxBlocks * kNoAllocWarpsPerBlock <= kMaxTrainWarps,
               "the train launcher must not cap the grid below one ray per warp");
 constexpr size_t kCounterOffset = (size_t)kNoAllocMaxBlocks * sizeof(double);
-constexpr size_t kScratchBytes = kCounterOffset + 256;
+constexpr size_t kScratchBytes = kCounterOffset + kTrainStateOffset + kTrainStateBytes;
 
-// The scratch: block loss partials, then the block counter. Every GPU that loads the
+// The scratch: block loss partials (fp64), the block counter, the state of an fp32 launch. Every GPU that loads the
 // library holds it until the process exits; every call shares it.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -65,6 +65,7 @@ int launch_noalloc(const pgb_grid* g, const pgb_rays* r, const void* target, dou
   a.loss_out = (Real*)loss_out;
   a.partials = (double*)scratch;
   a.counter = (unsigned*)(scratch + kCounterOffset);
+  a.state = (TrainState*)(scratch + kCounterOffset + kTrainStateOffset);
   a.loss_w = loss_weight;
   a.inv_count = r->num_rays > 0 ? 1.0 / (4.0 * (double)r->num_rays) : std::nan("");
   return dispatch_render<Real>(g, r, a, kTrain, stream);
@@ -90,9 +91,10 @@ extern "C" int pgb_render_train_noalloc(const pgb_grid* grid, const pgb_rays* ra
 
   void* scratch = nullptr;
   if ((st = scratch_address(&scratch))) return st;
-  // the block counter must start at zero; every partial is written before it is read
-  if (cudaMemsetAsync((unsigned char*)scratch + kCounterOffset, 0, sizeof(unsigned), stream) !=
-      cudaSuccess)
+  // the block counter and the launch state must start at zero; every partial is written
+  // before it is read
+  if (cudaMemsetAsync((unsigned char*)scratch + kCounterOffset, 0, kTrainStateOffset + kTrainStateBytes,
+                      stream) != cudaSuccess)
     return PGB_ERR_LAUNCH;
   if (grid->dtype == PGB_F64)
     return launch_noalloc<double>(grid, rays, target, loss_weight, rgba_out, grad_cells, loss_out,

@@ -14,8 +14,11 @@ template <typename Real> struct RenderArgs;
 // Counts one kernel launch and converts the launch status into a PGB status.
 int after_launch();
 
-// Most warps the fused training kernel may use (size of its per-warp loss table).
+// Most warps the fused fp64 training kernel may use (size of its loss table).
 constexpr int kMaxTrainWarps = 32768;
+// Bytes behind the fp64 loss tables of a training workspace: the block counter (fp64), then
+// the state of an fp32 launch (TrainState).
+constexpr int kTrainStateOffset = 256, kTrainStateBytes = 1024;
 // Samples per chunk are 32 * K; a ray may span at most this many chunks.
 constexpr int kMaxChunks = 32;
 // Largest samples-per-ray the fused kernels accept.

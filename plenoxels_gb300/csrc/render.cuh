@@ -79,6 +79,40 @@ __host__ __device__ inline bool quick_grid(int X, int Y, int Z, float ox, float 
          pd >= 9.094947e-13f && pd <= 1.0995116e12f;
 }
 
+// A sum of fp32 numbers kept exactly, so that it comes out the same in whatever order rays
+// are taken: each term's 24-bit mantissa is added as an integer to the bin of its exponent
+// (bin b: exponents 8 b .. 8 b + 7, worth 2^(8 b - 150)), 31 bits a term in a 64-bit bin.
+// Lane b of a warp holds bin b; infinities and NaN are flags beside them.
+struct BinSum {
+  long long bin = 0;
+  unsigned special = 0u;  // bit 0: +inf, 1: -inf, 2: NaN
+  __device__ __forceinline__ void add(float x, int lane) {  // the same x in every lane
+    const uint32_t u = __float_as_uint(x), e = (u >> 23) & 0xffu, m = u & 0x7fffffu;
+    if (e == 0xffu) {
+      special |= m != 0u ? 4u : (u >> 31) ? 2u : 1u;
+      return;
+    }
+    const uint32_t ex = e != 0u ? e : 1u;
+    const long long t = (long long)(e != 0u ? m | 0x800000u : m) << (ex & 7u);
+    if ((uint32_t)lane == ex >> 3) bin += (u >> 31) ? -t : t;
+  }
+  // the value over all lanes' bins
+  __device__ __forceinline__ double value(int lane) const {
+    const double unit = __longlong_as_double((long long)(1023 + 8 * lane - 150) << 52);
+    const double sum = warp_sum((double)bin * unit);
+    const double inf = __longlong_as_double(0x7ff0000000000000ll);
+    if (special == 0u) return sum;
+    return (special & 4u) || (special & 3u) == 3u ? inf - inf : (special & 1u) ? inf : -inf;
+  }
+};
+
+// What the warps of a training launch share (fp32). All zero between launches.
+struct TrainState {
+  unsigned long long bins[2][kWarp];  // squared errors, beta terms
+  unsigned special[2];
+  unsigned blocks_done;
+};
+
 template <typename Real>
 struct RenderArgs {
   GridP<Real> g;
@@ -110,8 +144,9 @@ struct RenderArgs {
   Real* grad;
   uint32_t* grad_marks;  // optional: units of written gradient cells are marked here
   Real* loss_out;
-  double* partials;
+  double* partials;  // fp64: block loss partials, and the block counter
   unsigned* counter;
+  TrainState* state;  // fp32
   double loss_w;
   double inv_count;
   // beta loss of scripts/train.py:170-177: beta_w * mean over all R*S samples of
@@ -667,37 +702,26 @@ __device__ __forceinline__ void warp_merged_scatter(const GridP<Real>& g, Real* 
   }
 }
 
-// Tuning knobs (compile-time; the shipped values are the measured best on GB300).
+// Blocks of the render kernels (compile-time; the shipped values are the measured best on
+// GB300). fp32 blocks share a queue of rays, so they are large: the fewer there are, the less
+// the slowest one waits for. Nearest lookup runs one block of 32 warps per SM (64 registers;
+// two of 16 warps took 76 us for 71 at 7500 rays x 600, 85 before the queue); trilinear
+// lookup with 32-sample chunks two blocks of 12 warps for the gradient (80 registers; one of
+// 24 warps the same within 2 %, six of 4 warps 345 us for 333) and two of 14 for a forward
+// pass (72 registers). Longer trilinear chunks need 90 to 210 registers: 8 warps a block, as
+// many blocks as fit. fp64 launches have a ray per warp, in blocks of 4 or 8 warps.
 #ifndef PGB_RENDER_THREADS
 #define PGB_RENDER_THREADS 256
 #endif
-#ifndef PGB_RENDER_MIN_BLOCKS
-#define PGB_RENDER_MIN_BLOCKS 0
+#ifndef PGB_RENDER_THREADS_NEAREST
+#define PGB_RENDER_THREADS_NEAREST 1024
 #endif
-// Nearest lookup (one load per sample) gains from more resident warps even at 64
-// registers with spills: 4 blocks per SM measured 0.0697 ms against 0.0765 ms at 2.
-#ifndef PGB_RENDER_MIN_BLOCKS_NEAREST
-#define PGB_RENDER_MIN_BLOCKS_NEAREST 4
-#endif
-// Trilinear lookup with 32-sample chunks: 24 resident warps per SM (80 registers, a
-// 32-byte spill) measured 0.127 ms per step against 0.133 ms at 16 (256^3, 8192 rays x
-// 256). Its blocks are 128 threads: a block holds its SM slot until its slowest ray ends,
-// and rays end at very different depths once they stop behind opaque cells, so smaller
-// blocks free slots sooner (kernel 0.094 ms against 0.098 ms at 256 threads; 64 threads
-// took 0.102 ms). Nearest lookup measured best at 256 threads.
 #ifndef PGB_RENDER_THREADS_K1
-#define PGB_RENDER_THREADS_K1 128
+#define PGB_RENDER_THREADS_K1 384
 #endif
-#ifndef PGB_RENDER_MIN_BLOCKS_K1
-#define PGB_RENDER_MIN_BLOCKS_K1 (3 * 256 / PGB_RENDER_THREADS_K1)
+#ifndef PGB_RENDER_THREADS_FWD
+#define PGB_RENDER_THREADS_FWD 448
 #endif
-
-constexpr int kRenderThreads = PGB_RENDER_THREADS;
-constexpr int kRenderThreadsK1 = PGB_RENDER_THREADS_K1;
-// the smallest block of any render launch (it bounds the number of blocks per ray count)
-constexpr int kRenderMinThreads = kRenderThreads < kRenderThreadsK1 ? kRenderThreads
-                                                                     : kRenderThreadsK1;
-
 
 // The per-warp shared-memory stage of the render and batched kernels: per chunk slot,
 // for the last M chunks,
@@ -917,21 +941,30 @@ constexpr int render_smem_bytes(int warps_per_block) {
   return RenderStage<Real, K, LOGT>::kBytesPerWarp * warps_per_block;
 }
 
-template <int MODE, int K>
+// the smallest block of an fp64 launch (it bounds the number of blocks per ray count)
+constexpr int kRenderMinThreads64 = 128;
+
+template <typename Real, int MODE, int K, int PHASE>
 constexpr int render_threads() {
-  return MODE != PGB_NEAREST && K == 1 ? kRenderThreadsK1 : kRenderThreads;
+  return sizeof(Real) != 4 ? (MODE != PGB_NEAREST && K == 1 ? kRenderMinThreads64 : PGB_RENDER_THREADS)
+         : MODE == PGB_NEAREST ? PGB_RENDER_THREADS_NEAREST
+         : K != 1 ? PGB_RENDER_THREADS
+         : PHASE == kForward ? PGB_RENDER_THREADS_FWD : PGB_RENDER_THREADS_K1;
 }
 
-template <int MODE, int K>
+template <typename Real, int MODE, int K, int PHASE>
 constexpr int render_min_blocks() {
-  return MODE == PGB_NEAREST ? PGB_RENDER_MIN_BLOCKS_NEAREST
-                             : (K == 1 ? PGB_RENDER_MIN_BLOCKS_K1 : PGB_RENDER_MIN_BLOCKS);
+  if (sizeof(Real) != 4) return MODE == PGB_NEAREST ? 4 : (K == 1 ? 6 : 0);
+  return MODE == PGB_NEAREST ? 1024 / PGB_RENDER_THREADS_NEAREST
+         : K != 1 ? 0
+         : PHASE == kForward ? 896 / PGB_RENDER_THREADS_FWD : 768 / PGB_RENDER_THREADS_K1;
 }
 
 // LOGT: transmittance as the compensated log-sum (scan_chunk_log, fp32 only) instead of
 // the reference's product scan. A: the index arithmetic (Arith).
 template <typename Real, typename Store, int MODE, int K, int PHASE, bool LOGT, int A>
-__global__ void __launch_bounds__((render_threads<MODE, K>()), (render_min_blocks<MODE, K>()))
+__global__ void __launch_bounds__((render_threads<Real, MODE, K, PHASE>()),
+                                  (render_min_blocks<Real, MODE, K, PHASE>()))
 render_kernel(const RenderArgs<Real> a) {
   static_assert(!LOGT || sizeof(Real) == 4, "log-sum transmittance is an fp32 form");
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -941,8 +974,20 @@ render_kernel(const RenderArgs<Real> a) {
   const int64_t gw = (int64_t)blockIdx.x * warps_per_block + (threadIdx.x >> 5);
   const int64_t nw = (int64_t)gridDim.x * warps_per_block;
   RenderStage<Real, K, LOGT> cs(smem_raw, threadIdx.x >> 5);
-  LossSum<Real> loss_lane;  // lane 0: squared errors of the warp's rays
-  LossSum<Real> beta_lane;  // per lane: beta terms of its samples
+  // Launches over fp32 grids are one wave of blocks whose warps each take the block's next ray
+  // when their last one ends (a counter in shared memory; block b has rays b, b + blocks, ...,
+  // so every block's rays come from all over the batch). With a ray per warp and 4 to 8 rays
+  // per block a slot waited for its slowest ray: 13 of 24 resident warps were busy on
+  // average. One training launch, before -> now: 256^3 trilinear, 8192 rays x 256, opaque
+  // blobs 79 -> 68 us; half transparent, 7500 rays x 600: trilinear 356 -> 333, nearest 131 ->
+  // 122 us; nearest, opaque 43 -> 36 us. A counter in global memory was slower (96 us for the
+  // first): its answers queue behind the gradient's atomics, and fetched a ray ahead they
+  // hand rays to warps that are still busy.
+  constexpr bool QUEUE = sizeof(Real) == 4;
+  constexpr bool SUMS = QUEUE && PHASE == kTrain;  // loss sums that no order of rays changes
+  BinSum loss_bins, beta_bins;  // SUMS
+  LossSum<Real> loss_lane;  // otherwise, lane 0: squared errors of the warp's rays
+  LossSum<Real> beta_lane;  // per lane: beta terms of its samples (SUMS: of the current ray)
   const bool with_beta = PHASE == kTrain && a.use_beta;
   // Exact early stop. With alpha clamped to [0,1], T is exactly 0 only behind an opaque
   // sample z (alpha_z = 1) or after an underflow, and every later sample then has weight
@@ -960,12 +1005,27 @@ render_kernel(const RenderArgs<Real> a) {
   __shared__ double s_part[32];  // per-warp loss partials (training phase)
   __shared__ double s_part_beta[32];
   __shared__ unsigned s_done;    // warps of this block that finished (training phase)
-  if (PHASE == kTrain) {
-    if (threadIdx.x == 0) s_done = 0u;
+  __shared__ unsigned long long s_bins[2][kWarp];  // SUMS: the block's sums
+  __shared__ unsigned s_special[2];
+  __shared__ unsigned s_taken;  // QUEUE: rays of this block that have a warp
+  if (QUEUE || PHASE == kTrain) {
+    if (threadIdx.x == 0) {
+      s_done = 0u;
+      s_taken = (unsigned)warps_per_block;
+    }
+    if (SUMS && threadIdx.x < 2 * kWarp) s_bins[threadIdx.x >> 5][lane] = 0ull;
+    if (SUMS && threadIdx.x < 2) s_special[threadIdx.x] = 0u;
     __syncthreads();
   }
+  const auto next_ray = [&](int64_t r) -> int64_t {
+    if (!QUEUE) return r + nw;
+    unsigned taken = 0;
+    if (lane == 0) taken = atomicAdd(&s_taken, 1u);
+    return (int64_t)blockIdx.x + (int64_t)gridDim.x * __shfl_sync(kFull, taken, 0);
+  };
 
-  for (int64_t r = gw; r < a.R; r += nw) {
+  for (int64_t r = QUEUE ? (int64_t)blockIdx.x + (int64_t)gridDim.x * (threadIdx.x >> 5) : gw; r < a.R;
+       r = next_ray(r)) {
     Ray<Real> ray;
     load_ray(a, r, ray, PHASE == kTrain);
     int first, end;
@@ -976,6 +1036,7 @@ render_kernel(const RenderArgs<Real> a) {
       end = with_beta ? a.S : end;
     }
     const int nchunks = (end - first + kWarp * K - 1) / (kWarp * K);
+    if (SUMS) beta_lane = LossSum<Real>();
     if (with_beta && lane == 0 && end - first < a.S)  // the samples left out have alpha 0
       beta_lane.add((Real)(a.S - (end - first)) * a.beta_zero);
 
@@ -1074,7 +1135,16 @@ render_kernel(const RenderArgs<Real> a) {
         sq += diff * diff;
         gpx[ch] = grad_scale * diff;
       }
-      if (lane == 0) loss_lane.add(sq);
+      if constexpr (SUMS) {
+        loss_bins.add(sq, lane);
+        if (with_beta) {
+          const LossSum<Real> ray_beta = warp_sum(beta_lane);
+          beta_bins.add(__shfl_sync(kFull, ray_beta.hi, 0), lane);
+          beta_bins.add(__shfl_sync(kFull, ray_beta.lo, 0), lane);
+        }
+      } else {
+        if (lane == 0) loss_lane.add(sq);
+      }
       if (a.rgba_out != nullptr && lane < 4) a.rgba_out[4 * r + lane] = pick4(px, lane);
     }
     if (a.use_bg)  // d(rgb + (1 - A) bg)/dA = -bg
@@ -1154,7 +1224,52 @@ render_kernel(const RenderArgs<Real> a) {
     }
   }
 
-  if (PHASE == kTrain) {
+  if constexpr (SUMS) {
+    // Warps add their bins up in shared memory and the block's last warp adds them to the
+    // launch's, so that a block fences once, at its end (a fence at device scope also empties
+    // the SM's L1: one per warp took the nearest step of 8192 rays from 44 to 66 us). The last
+    // block takes the sums and leaves the state zero for the next launch.
+    TrainState* st = a.state;
+    if (loss_bins.bin != 0) atomicAdd(&s_bins[0][lane], (unsigned long long)loss_bins.bin);
+    if (beta_bins.bin != 0) atomicAdd(&s_bins[1][lane], (unsigned long long)beta_bins.bin);
+    if (lane == 0) {
+      if (loss_bins.special) atomicOr(&s_special[0], loss_bins.special);
+      if (beta_bins.special) atomicOr(&s_special[1], beta_bins.special);
+    }
+    __threadfence_block();
+    __syncwarp();
+    unsigned last = 0;
+    if (lane == 0) last = atomicAdd(&s_done, 1u) == (unsigned)warps_per_block - 1u;
+    if (!__shfl_sync(kFull, last, 0)) return;
+    __threadfence_block();
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const unsigned long long bin = *(volatile unsigned long long*)&s_bins[i][lane];
+      const unsigned special = *(volatile unsigned*)&s_special[i];
+      if (bin != 0ull) atomicAdd(&st->bins[i][lane], bin);
+      if (lane == 0 && special != 0u) atomicOr(&st->special[i], special);
+    }
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) last = atomicAdd(&st->blocks_done, 1u) == gridDim.x - 1u;
+    if (!__shfl_sync(kFull, last, 0)) return;
+    __threadfence();
+    BinSum sums[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      sums[i].bin = (long long)__ldcg(&st->bins[i][lane]);
+      sums[i].special = __ldcg(&st->special[i]);
+    }
+    const double mse = sums[0].value(lane), beta = with_beta ? sums[1].value(lane) : 0.0;
+    st->bins[0][lane] = 0ull;
+    st->bins[1][lane] = 0ull;
+    if (lane == 0) {
+      a.loss_out[0] = (Real)(a.loss_w * mse * a.inv_count);
+      if (with_beta) a.loss_out[1] = (Real)(a.beta_w * beta * a.inv_samples);
+      st->blocks_done = 0u;
+      st->special[0] = st->special[1] = 0u;
+    }
+  } else if (PHASE == kTrain) {
     // deterministic loss without a barrier: warps count themselves out in shared memory,
     // the block's last warp sums the block in warp order and takes one global ticket, and
     // the last block sums the blocks in block order

@@ -13,23 +13,36 @@ namespace pgb {
 
 template <typename Real, typename Store, int MODE, int K, int PHASE, bool LOGT, int A>
 int launch_render_k(const RenderArgs<Real>& a, cudaStream_t s) {
-  constexpr int kThreads = render_threads<MODE, K>();
+  constexpr int kThreads = render_threads<Real, MODE, K, PHASE>();
   constexpr int kWarpsPerBlock = kThreads / kWarp;
   constexpr int kSmem = render_smem_bytes<Real, K, LOGT>(kWarpsPerBlock);
   // the dynamic shared-memory opt-in (dynamic + static may pass 48 KiB) is per device:
-  // set it on first use of each device
+  // set it on first use of each device, and note how many blocks the device holds
   static int configured[64] = {0};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && !configured[dev]) {
+  int resident = dev >= 0 && dev < 64 ? configured[dev] : 0;
+  if (resident == 0) {
     if (cudaFuncSetAttribute(render_kernel<Real, Store, MODE, K, PHASE, LOGT, A>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess)
       return PGB_ERR_LAUNCH;
-    configured[dev] = 1;
+    int sms = 0, per_sm = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &per_sm, render_kernel<Real, Store, MODE, K, PHASE, LOGT, A>, kThreads, kSmem) !=
+            cudaSuccess ||
+        sms * per_sm < 1)
+      return PGB_ERR_LAUNCH;
+    resident = sms * per_sm;
+    if (dev >= 0 && dev < 64) configured[dev] = resident;
   }
-  int64_t blocks = (a.R + kWarpsPerBlock - 1) / kWarpsPerBlock;
-  blocks = std::min<int64_t>(blocks, PHASE == kTrain ? kMaxTrainWarps / kWarpsPerBlock
-                                                     : (int64_t)1 << 20);
+  // fp32: one wave, or a ray per block when there are fewer rays; fp64: a ray per warp
+  int64_t blocks = a.R;
+  if (sizeof(Real) == 4)
+    blocks = std::min<int64_t>(blocks, resident);
+  else
+    blocks = std::min<int64_t>((a.R + kWarpsPerBlock - 1) / kWarpsPerBlock,
+                               PHASE == kTrain ? kMaxTrainWarps / kWarpsPerBlock : (int64_t)1 << 20);
   if (blocks < 1) blocks = 1;
   render_kernel<Real, Store, MODE, K, PHASE, LOGT, A><<<(unsigned)blocks, kThreads, kSmem, s>>>(a);
   return after_launch();
