@@ -11,10 +11,9 @@
 //  pgb_adam_tv_step  the two passes above fused: Adam on grad + the TV gradient, written
 //                to a second parameter buffer
 #include <algorithm>
-#include <cmath>
 
 #include "pgb_host.h"
-#include "pgb_device.cuh"
+#include "adam.cuh"
 
 namespace pgb {
 namespace {
@@ -142,37 +141,33 @@ __global__ void __launch_bounds__(kTvThreads) tv_grad_kernel(const float4* __res
   }
 }
 
-struct AdamConst {
-  float one_minus_b1, b2, one_minus_b2, step_size, inv_bc2_sqrt, eps;
-};
-
-__device__ __forceinline__ float adam_one(float& p, float g, float& m, float& s, const AdamConst& k) {
-  m = m + k.one_minus_b1 * (g - m);        // exp_avg.lerp_(grad, 1 - beta1)
-  s = s * k.b2 + k.one_minus_b2 * g * g;   // exp_avg_sq.mul_(beta2).addcmul_(grad, grad, 1 - beta2)
-  const float denom = sqrtf(s) * k.inv_bc2_sqrt + k.eps;
-  p = p - k.step_size * (m / denom);
-  return fabsf(g);
-}
-
-__global__ void adam_kernel(float4* __restrict__ p, float4* __restrict__ g, float4* __restrict__ m,
-                            float4* __restrict__ s, float4* __restrict__ acc, int64_t n4,
-                            AdamConst k, int zero_grad) {
+// Adam's bytes per cell depend on what the step touched. The gradient and the moments are
+// read first. A cell with gradient and moments 0 (no ray has reached it yet) stays as it is,
+// bit for bit: 48 bytes instead of 160. A cell without a gradient in this step (most of the
+// grid: a step's rays cross a few per cent to a third of the cells) leaves |grad| and the
+// zeroed gradient alone: 112 bytes. Lanes decide each for itself; sectors hold two cells.
+// Bound by HBM. 256^3, 7500 rays x 600 nearest, half of the cells seen so far: 411 -> 246 us;
+// 192^3 173 -> 114 us; every cell with a gradient 360 -> 352 us. The second round of loads
+// waits for the first, so it wants many warps: 48 per SM (40 registers); 40 or 56 warps took
+// 281 and 296 us, two cells per thread (78 registers) 350 us, evict-first accesses 312 us.
+__global__ void __launch_bounds__(256, 6) adam_kernel(float4* __restrict__ p, float4* __restrict__ g,
+                                                      float4* __restrict__ m, float4* __restrict__ s,
+                                                      float4* __restrict__ acc, int64_t n4, AdamConst k,
+                                                      int zero_grad) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4;
        i += (int64_t)gridDim.x * blockDim.x) {
-    float4 P = p[i], Gr = g[i], M = m[i], S = s[i];
-    float4 A = make_float4(0.f, 0.f, 0.f, 0.f);
-    A.x = adam_one(P.x, Gr.x, M.x, S.x, k);
-    A.y = adam_one(P.y, Gr.y, M.y, S.y, k);
-    A.z = adam_one(P.z, Gr.z, M.z, S.z, k);
-    A.w = adam_one(P.w, Gr.w, M.w, S.w, k);
+    const float4 G = g[i];
+    float4 M = m[i], S = s[i];
+    const bool touched = any_nonzero(G);
+    if (!touched && k.rest_stays && !any_nonzero(M) && !any_nonzero(S)) continue;
+    float4 P = p[i], A = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (touched && acc) A = acc[i];
+    const float4 d = adam_cell(P, G, M, S, k);
     p[i] = P;
     m[i] = M;
     s[i] = S;
-    if (acc) {
-      float4 a = acc[i];
-      a.x += A.x; a.y += A.y; a.z += A.z; a.w += A.w;
-      acc[i] = a;
-    }
+    if (!touched) continue;
+    if (acc) acc[i] = add4(A, d);
     if (zero_grad) g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
 }
@@ -181,8 +176,10 @@ __global__ void adam_kernel(float4* __restrict__ p, float4* __restrict__ g, floa
 // order, same fp32 expression) feeding adam_one, over the (z-blocks, Y, x-chunks) grid of
 // the TV kernels. Neighbours are read from pin while cells are updated, so the update goes
 // to pout (a different buffer): one pass instead of the TV gradient's read-modify-write of
-// grad followed by Adam.
-__global__ void __launch_bounds__(kTvThreads) adam_tv_kernel(
+// grad followed by Adam. Every cell has a TV gradient, so only the zeroing of the render
+// step's gradient depends on what that touched. Bound by HBM, 160 bytes a cell: 256^3 433 ->
+// 396 us, with 40 warps per SM (48 registers; at 55 registers and 32 warps 454 us).
+__global__ void __launch_bounds__(kTvThreads, 5) adam_tv_kernel(
     const float4* __restrict__ pin, float4* __restrict__ pout, float4* __restrict__ g,
     float4* __restrict__ mo, float4* __restrict__ so, float4* __restrict__ acc, int X, int Y,
     int Z, const double* __restrict__ sumsq, float weight, AdamConst k, int zero_grad) {
@@ -200,6 +197,7 @@ __global__ void __launch_bounds__(kTvThreads) adam_tv_kernel(
   for (int x = x0; x < x1; ++x, i += YZ) {
     const float4 next = x + 1 < X ? __ldg(pin + i + YZ) : m;
     float4 Gr = g[i];
+    const bool written = any_nonzero(Gr);  // by the render step; else it is 0 already
     if (tv) {
       float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
       auto add = [&](float4 nb) {
@@ -214,41 +212,19 @@ __global__ void __launch_bounds__(kTvThreads) adam_tv_kernel(
       Gr.x += c * d.x; Gr.y += c * d.y; Gr.z += c * d.z; Gr.w += c * d.w;
     }
     float4 P = m, M = mo[i], S = so[i];
-    float4 A;
-    A.x = adam_one(P.x, Gr.x, M.x, S.x, k);
-    A.y = adam_one(P.y, Gr.y, M.y, S.y, k);
-    A.z = adam_one(P.z, Gr.z, M.z, S.z, k);
-    A.w = adam_one(P.w, Gr.w, M.w, S.w, k);
+    const float4 A = adam_cell(P, Gr, M, S, k);
     pout[i] = P;
     mo[i] = M;
     so[i] = S;
-    if (acc) {
-      float4 a = acc[i];
-      a.x += A.x; a.y += A.y; a.z += A.z; a.w += A.w;
-      acc[i] = a;
-    }
-    if (zero_grad) g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (acc) acc[i] = add4(acc[i], A);
+    if (zero_grad && written) g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     prev = m;
     m = next;
   }
 }
 
-AdamConst adam_const(double lr, double beta1, double beta2, double eps, int64_t step) {
-  // torch.optim.Adam (non-capturable path): bias corrections in double on the host
-  const double bc1 = 1.0 - std::pow(beta1, (double)step);
-  const double bc2 = 1.0 - std::pow(beta2, (double)step);
-  AdamConst k;
-  k.one_minus_b1 = (float)(1.0 - beta1);
-  k.b2 = (float)beta2;
-  k.one_minus_b2 = (float)(1.0 - beta2);
-  k.step_size = (float)(lr / bc1);
-  k.inv_bc2_sqrt = (float)(1.0 / std::sqrt(bc2));
-  k.eps = (float)eps;
-  return k;
-}
-
 inline unsigned stream_blocks(int64_t n) {
-  return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 152 * 16));
+  return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 152 * 48));
 }
 
 inline bool al16(const void* p) { return ((uintptr_t)p % 16) == 0; }
