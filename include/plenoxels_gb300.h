@@ -277,6 +277,13 @@ int pgb_avg_pool3d_fwd(const float* cells, const int32_t dims[3], int32_t window
  * is needed). */
 int pgb_avg_pool3d_bwd(const float* d_out, const int32_t dims[3], int32_t window, int32_t stride,
                        void* scratch, float* d_cells, pgb_stream_t stream);
+/* pgb_avg_pool3d_bwd followed by pgb_adam_step on its result (scripts/train.py:108-123, 181-184
+ * while progressive growing runs), without the full gradient in memory. param, exp_avg,
+ * exp_avg_sq and abs_grad_accum (optional) are [X,Y,Z,4]. */
+int pgb_avg_pool3d_bwd_adam(const float* d_out, const int32_t dims[3], int32_t window, int32_t stride,
+                            void* scratch, float* param, float* exp_avg, float* exp_avg_sq,
+                            float* abs_grad_accum, double lr, double beta1, double beta2, double eps,
+                            int64_t step, pgb_stream_t stream);
 
 /* ---- drop-in operators, one per reference function ---- */
 

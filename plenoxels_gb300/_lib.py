@@ -115,6 +115,8 @@ _SIGNATURES = {
     "pgb_avg_pool3d_shape": (c_int32, [POINTER(c_int32), c_int32, c_int32, POINTER(c_int32), POINTER(c_int64)]),
     "pgb_avg_pool3d_fwd": (c_int32, [_P, POINTER(c_int32), c_int32, c_int32, _P, _P, _P]),
     "pgb_avg_pool3d_bwd": (c_int32, [_P, POINTER(c_int32), c_int32, c_int32, _P, _P, _P]),
+    "pgb_avg_pool3d_bwd_adam": (c_int32, [_P, POINTER(c_int32), c_int32, c_int32, _P, _P, _P, _P, _P, c_double,
+                                          c_double, c_double, c_double, c_int64, _P]),
     "pgb_generate_rays": (c_int32, [_P, c_int32, c_int64, c_float, _P, c_int32, c_int32, _P, c_int32, _P, _P, _P, _P]),
     "pgb_sample_points": (c_int32, [_P, c_int32, c_int64, _P, c_int32, c_float, _P, _P]),
     "pgb_coords_min": (c_int32, [_P, c_int64, _P, _P]),

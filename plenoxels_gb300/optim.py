@@ -59,6 +59,19 @@ class FusedAdam:
                                         self.step_count, 1 if zero_grad else 0, s), "adam step")
 
     @torch.no_grad()
+    def step_pooled(self, pooled_grad, window, stride, scratch):
+        """step on the gradient of average_pool3d_grid's input, given its output's gradient
+        [Xo,Yo,Zo,4]: the pooling's adjoint and the update in one pass over the grid, without
+        the full gradient in memory. scratch: the bytes of grid_functions.pool_shape."""
+        g = self.grid
+        self.step_count += 1
+        s = torch.cuda.current_stream(g.device).cuda_stream
+        check(_lib.load().pgb_avg_pool3d_bwd_adam(
+            ptr(pooled_grad), _lib.dims3(g.shape), window, stride, ptr(scratch), ptr(g), ptr(self.exp_avg),
+            ptr(self.exp_avg_sq), ptr(self.abs_grad), self.lr, self.betas[0], self.betas[1], self.eps,
+            self.step_count, s), "pooled adam step")
+
+    @torch.no_grad()
     def step_tv(self, grad, weight, out, zero_grad=True):
         """add_tv on the optimised grid followed by step, in two passes instead of three:
         the TV loss value (one reduction over the grid), then Adam on grad + the TV gradient

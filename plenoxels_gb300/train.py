@@ -13,8 +13,8 @@ place, at the cost of the separate TV gradient pass).
 Progressive growing (scripts/train.py:91-123): while the schedule's receptive field r is
 above 1, the step renders the grid average-pooled with window r and stride max(1, r//4)
 (pitch points_distance * stride, origin at the coordinate of cell r//2), and the pooled
-gradient is spread back onto the full grid by the pooling's adjoint, which rewrites the
-whole full gradient. The TV term applies once r < 19, to the grid being rendered.
+gradient is spread back onto the full grid by the pooling's adjoint inside the Adam pass
+(the full gradient stays zero). The TV term applies once r < 19, to the grid being rendered.
 """
 from __future__ import annotations
 
@@ -54,6 +54,8 @@ class Trainer:
         self.step_index = 0
         self._pooled = {}  # field -> (pooled grid, its FusedTrainStep, stride, scratch)
         self.losses = torch.zeros(3, device=grid.device)  # mse, tv, beta of the last step
+        # the full gradient is all zeros between steps, unless the caller writes to it
+        self._grad_version = self.render.grad._version
 
     def field(self, i):
         """Receptive field of step i (scripts/train.py:108); 0 once the schedule ends."""
@@ -106,10 +108,14 @@ class Trainer:
             return self.losses
         if self.tv > 0.0 and r < 19:
             self.losses[1] = self.opt.add_tv(tv_grad, self.tv, grid=tv_grid)
-        if r > 1:
-            check(lib.pgb_avg_pool3d_bwd(ptr(render_step.grad), _lib.dims3(self.grid.shape), r,
-                                         stride, ptr(scratch), ptr(full_grad), s), "pooled grid")
-        self.opt.step(full_grad)
+        if r > 1 and full_grad._version == self._grad_version:
+            self.opt.step_pooled(render_step.grad, r, stride, scratch)
+        else:
+            if r > 1:  # the caller wrote to the full gradient: the step overwrites and zeroes it
+                check(lib.pgb_avg_pool3d_bwd(ptr(render_step.grad), _lib.dims3(self.grid.shape), r,
+                                             stride, ptr(scratch), ptr(full_grad), s), "pooled grid")
+                self._grad_version = full_grad._version
+            self.opt.step(full_grad)
         self.step_index += 1
         return self.losses
 
