@@ -399,6 +399,11 @@ int pgb_splat_preview(const float* cells, const int32_t dims[3], float points_di
  * cleared. kernel_size odd and <= 7; sums_scratch holds X*Y*Z floats. */
 int pgb_remove_noise(float* cells, const int32_t dims[3], int32_t kernel_size, double radius,
                      float threshold, int32_t repeats, float* sums_scratch, pgb_stream_t stream);
+/* The same, faster, with pgb_remove_noise_scratch_bytes(dims, repeats) bytes of scratch (16-byte
+ * aligned): repeats run on two planes of alphas, and stop once one changes none. */
+int64_t pgb_remove_noise_scratch_bytes(const int32_t dims[3], int32_t repeats);
+int pgb_remove_noise_planes(float* cells, const int32_t dims[3], int32_t kernel_size, double radius,
+                            float threshold, int32_t repeats, void* scratch, pgb_stream_t stream);
 
 /* Zero `bytes` bytes at ptr (16-byte aligned) with a vectorised store kernel: the
  * gradient zeroing of optimizer.zero_grad() (scripts/train.py:180) and of a fresh .grad. */

@@ -141,6 +141,8 @@ _SIGNATURES = {
     "pgb_splat_preview": (c_int32, [_P, POINTER(c_int32), c_float, POINTER(c_float), c_float, c_int32, c_float,
                                     _P, _P, _P]),
     "pgb_remove_noise": (c_int32, [_P, POINTER(c_int32), c_int32, c_double, c_float, c_int32, _P, _P]),
+    "pgb_remove_noise_scratch_bytes": (c_int64, [POINTER(c_int32), c_int32]),
+    "pgb_remove_noise_planes": (c_int32, [_P, POINTER(c_int32), c_int32, c_double, c_float, c_int32, _P, _P]),
     "pgb_hash_uniform": (c_float, [c_uint64, c_uint64, c_uint32]),
     "pgb_launch_count": (c_int64, []),
     "pgb_version": (c_char_p, []),
