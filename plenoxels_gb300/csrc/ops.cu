@@ -22,6 +22,13 @@ inline unsigned blocks_for(int64_t n, int per_thread = 1) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (n);     \
        i += (int64_t)gridDim.x * blockDim.x)
 
+// a / b for non-negative a and positive b, in 32 bits where both fit (a 64-bit division is a
+// hundred instructions).
+__device__ __forceinline__ int64_t quotient(int64_t a, int64_t b) {
+  if (((a | b) >> 32) == 0) return (int64_t)((uint32_t)a / (uint32_t)b);
+  return a / b;
+}
+
 // --------------------------------------------------------------- ray generation
 // src/ray_sampling.py:195-264. One thread per ray (camera-major).
 __global__ void generate_rays_kernel(const float* __restrict__ T, int C, int64_t Rc, float fov,
@@ -78,9 +85,9 @@ __global__ void sample_points_kernel(const float* __restrict__ T, int64_t Rc, in
                                      const float* __restrict__ dirs, float delta, int64_t total,
                                      float* __restrict__ out) {
   PGB_FOR(i, total) {
-    const int64_t r = i / S;
+    const int64_t r = quotient(i, S);
     const int k = (int)(i - r * S) + 1;
-    const int c = (int)(r / Rc);
+    const int c = (int)quotient(r, Rc);
     const float t = rmul(delta, (float)k);
     const float* P = T + 16 * (int64_t)c;
     out[3 * i + 0] = radd(P[3], rmul(dirs[3 * r + 0], t));
@@ -109,7 +116,17 @@ __global__ void min_init_kernel(int* out) {
 __global__ void __launch_bounds__(kThreads) coords_min_kernel(const float* __restrict__ coords,
                                                               int64_t count, int* out) {
   float m[3] = {__int_as_float(0x7f800000), __int_as_float(0x7f800000), __int_as_float(0x7f800000)};
-  PGB_FOR(i, count) {
+  // four coordinates are three 16-byte words (when the table is 16-byte aligned)
+  const int64_t fours = (reinterpret_cast<uintptr_t>(coords) & 15u) == 0 ? count / 4 : 0;
+  const float4* words = reinterpret_cast<const float4*>(coords);
+  PGB_FOR(i, fours) {
+    const float4 a = __ldg(words + 3 * i), b = __ldg(words + 3 * i + 1), c = __ldg(words + 3 * i + 2);
+    m[0] = fminf(fminf(m[0], fminf(a.x, a.w)), fminf(b.z, c.y));
+    m[1] = fminf(fminf(m[1], fminf(a.y, b.x)), fminf(b.w, c.z));
+    m[2] = fminf(fminf(m[2], fminf(a.z, b.y)), fminf(c.x, c.w));
+  }
+  for (int64_t i = 4 * fours + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count;
+       i += (int64_t)gridDim.x * blockDim.x) {
 #pragma unroll
     for (int a = 0; a < 3; ++a) m[a] = fminf(m[a], __ldg(coords + 3 * i + a));
   }
@@ -143,14 +160,25 @@ __global__ void min_finish_kernel(int* out) {
   }
 }
 
-// src/ray_sampling.py:13
-__global__ void normalize_kernel(const float* __restrict__ samples, int64_t count,
+// src/ray_sampling.py:13. Four coordinates (three 16-byte words) per thread where both
+// tables are aligned; `fours` of them, the rest one by one.
+__global__ void normalize_kernel(const float* __restrict__ samples, int64_t count, int64_t fours,
                                  const float* __restrict__ gmin, float pd, float* __restrict__ out) {
   const float m0 = gmin[0], m1 = gmin[1], m2 = gmin[2];
-  PGB_FOR(i, count) {
-    out[3 * i + 0] = rdiv(rsub(samples[3 * i + 0], m0), pd);
-    out[3 * i + 1] = rdiv(rsub(samples[3 * i + 1], m1), pd);
-    out[3 * i + 2] = rdiv(rsub(samples[3 * i + 2], m2), pd);
+  const auto norm = [pd](float x, float m) { return rdiv(rsub(x, m), pd); };
+  const float4* in = reinterpret_cast<const float4*>(samples);
+  float4* to = reinterpret_cast<float4*>(out);
+  PGB_FOR(i, fours) {
+    const float4 a = __ldg(in + 3 * i), b = __ldg(in + 3 * i + 1), c = __ldg(in + 3 * i + 2);
+    to[3 * i] = make_float4(norm(a.x, m0), norm(a.y, m1), norm(a.z, m2), norm(a.w, m0));
+    to[3 * i + 1] = make_float4(norm(b.x, m1), norm(b.y, m2), norm(b.z, m0), norm(b.w, m1));
+    to[3 * i + 2] = make_float4(norm(c.x, m2), norm(c.y, m0), norm(c.z, m1), norm(c.w, m2));
+  }
+  for (int64_t i = 4 * fours + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    out[3 * i + 0] = norm(samples[3 * i + 0], m0);
+    out[3 * i + 1] = norm(samples[3 * i + 1], m1);
+    out[3 * i + 2] = norm(samples[3 * i + 2], m2);
   }
 }
 
@@ -228,24 +256,28 @@ __global__ void nearest_scatter_kernel(GridP<Real> g, const Real* __restrict__ n
 }
 
 // src/grid_functions.py:220-246: corners in the order x in {ceil, floor}, y in {ceil,
-// floor}, z in {ceil, floor}; not wrapped.
-template <typename Real>
-__global__ void corner_indices_kernel(const Real* __restrict__ n, int64_t count,
+// floor}, z in {ceil, floor}; not wrapped. A sample's 24 indices are 12 words of 16 bytes; a
+// thread makes one word, so that a warp's stores are contiguous (a thread per sample stored
+// at a stride of 192 bytes: 768,000 samples
+// 123 us, now 42; writing the words takes 22). PER: indices per
+// word, 1 for an output that is not 16-byte aligned.
+template <typename Real, int PER>
+__global__ void corner_indices_kernel(const Real* __restrict__ n, int64_t words,
                                       int64_t* __restrict__ out) {
-  PGB_FOR(i, count) {
-    long long c[3], f[3];
+  PGB_FOR(t, words) {
+    const int64_t i = quotient(t, 24 / PER);
+    const int e = PER * (int)(t - (24 / PER) * i);  // the word's first index: corner e / 3, axis e % 3
+    long long v[PER];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      c[a] = to_i64(rceil(n[3 * i + a]));
-      f[a] = to_i64(rfloor(n[3 * i + a]));
+    for (int u = 0; u < PER; ++u) {
+      const int corner = (e + u) / 3, ax = (e + u) - 3 * corner;
+      const Real x = __ldg(n + 3 * i + ax);
+      v[u] = to_i64((corner & (4 >> ax)) ? rfloor(x) : rceil(x));
     }
-#pragma unroll
-    for (int corner = 0; corner < 8; ++corner) {
-      int64_t* o = out + 24 * i + 3 * corner;
-      o[0] = (corner & 4) ? f[0] : c[0];
-      o[1] = (corner & 2) ? f[1] : c[1];
-      o[2] = (corner & 1) ? f[2] : c[2];
-    }
+    if constexpr (PER == 2)
+      reinterpret_cast<longlong2*>(out)[t] = make_longlong2(v[0], v[1]);
+    else
+      out[t] = v[0];
   }
 }
 
@@ -259,12 +291,27 @@ __global__ void in_bounds_kernel(const T* __restrict__ idx, int64_t count, int X
   }
 }
 
-// src/grid_functions.py:66-79
-__global__ void wrap_kernel(int64_t* __restrict__ idx, int64_t count, int X, int Y, int Z) {
-  PGB_FOR(i, count) {
-    idx[3 * i + 0] = floor_mod(idx[3 * i + 0], X);
-    idx[3 * i + 1] = floor_mod(idx[3 * i + 1], Y);
-    idx[3 * i + 2] = floor_mod(idx[3 * i + 2], Z);
+// src/grid_functions.py:66-79. Index e of the flat list belongs to axis e % 3; pairs are read
+// as 16-byte words, and only words with an index out of range are written back (a thread per
+// index triple read and wrote all of them at a stride of 24 bytes: 2.3 M triples
+// half out of range 78 us, now 50).
+__global__ void wrap_pairs_kernel(longlong2* __restrict__ idx, int64_t pairs, int X, int Y, int Z) {
+  PGB_FOR(t, pairs) {
+    const longlong2 v = idx[t];
+    const int a = (int)(2 * t - 3 * quotient(2 * t, 3));  // axis of the first
+    const int m0 = a == 0 ? X : a == 1 ? Y : Z, m1 = a == 0 ? Y : a == 1 ? Z : X;
+    if ((unsigned long long)v.x < (unsigned long long)m0 && (unsigned long long)v.y < (unsigned long long)m1)
+      continue;
+    idx[t] = make_longlong2(floor_mod(v.x, m0), floor_mod(v.y, m1));
+  }
+}
+
+// One index per thread, from index `from` on.
+__global__ void wrap_kernel(int64_t* __restrict__ idx, int64_t from, int64_t count, int X, int Y, int Z) {
+  PGB_FOR(t, count - from) {
+    const int64_t e = from + t;
+    const int a = (int)(e - 3 * quotient(e, 3));
+    idx[e] = floor_mod(idx[e], a == 0 ? X : a == 1 ? Y : Z);
   }
 }
 
@@ -291,69 +338,76 @@ __device__ __forceinline__ bool corner_cell(const GridP<Real>& g, const int64_t*
 template <typename Real>
 __device__ __forceinline__ Real frac_ref(Real x) { return rsub(x, rtrunc(x)); }
 
+// A thread per corner, eight lanes per sample: the corners' 192 bytes of indices and the cells
+// are read by neighbouring lanes, and the blend goes across them (corner bit 4: x, 2: y, 1: z;
+// the partner along an axis is the lane with that bit changed; products and sums are rounded
+// as the reference rounds them, and a sum does not depend on its operands' order). A thread
+// per sample read its indices at a stride of 192 bytes: 768,000
+// samples 74 us, now 54.
 template <typename Real, typename Store>
 __global__ void trilinear_gather_kernel(GridP<Real> g, const Real* __restrict__ n,
-                                        const int64_t* __restrict__ corners, int64_t count,
+                                        const int64_t* __restrict__ corners, int64_t lanes,
                                         Real* __restrict__ out, int* __restrict__ status) {
-  PGB_FOR(i, count) {
-    const Real wx = frac_ref(n[3 * i]), wy = frac_ref(n[3 * i + 1]), wz = frac_ref(n[3 * i + 2]);
-    const Real ux = rsub(Real(1), wx), uy = rsub(Real(1), wy), uz = rsub(Real(1), wz);
-    Real cv[8][4];
-#pragma unroll
-    for (int corner = 0; corner < 8; ++corner) {
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  const int64_t whole = (lanes + kWarp - 1) / kWarp * kWarp;  // whole warps take part in the shuffles
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < whole; t += step) {
+    const bool in = t < lanes;
+    const int64_t i = t >> 3;
+    const int corner = (int)t & 7;
+    Real v[4] = {Real(0), Real(0), Real(0), Real(0)};
+    Real w[3] = {Real(0), Real(0), Real(0)};
+    if (in) {
       uint64_t cell;
-      if (corner_cell(g, corners + 24 * i + 3 * corner, cell, status)) {
-        CellIO<Store>::load(g.cells, cell, cv[corner]);
-      } else {
-        cv[corner][0] = cv[corner][1] = cv[corner][2] = cv[corner][3] = Real(0);
-      }
+      if (corner_cell(g, corners + 3 * t, cell, status)) CellIO<Store>::load(g.cells, cell, v);
       if (g.clip) {
 #pragma unroll
-        for (int ch = 0; ch < 4; ++ch) cv[corner][ch] = clamp01(cv[corner][ch]);
+        for (int ch = 0; ch < 4; ++ch) v[ch] = clamp01(v[ch]);
+      }
+#pragma unroll
+      for (int ax = 0; ax < 3; ++ax) {
+        const Real f = frac_ref(__ldg(n + 3 * i + ax));
+        w[ax] = (corner & (4 >> ax)) ? rsub(Real(1), f) : f;
       }
     }
 #pragma unroll
-    for (int ch = 0; ch < 4; ++ch) {
-      Real a4[4];
+    for (int ax = 0; ax < 3; ++ax) {
 #pragma unroll
-      for (int yz = 0; yz < 4; ++yz) a4[yz] = radd(rmul(cv[yz][ch], wx), rmul(cv[4 + yz][ch], ux));
-      const Real b0 = radd(rmul(a4[0], wy), rmul(a4[2], uy));
-      const Real b1 = radd(rmul(a4[1], wy), rmul(a4[3], uy));
-      out[4 * i + ch] = radd(rmul(b0, wz), rmul(b1, uz));
+      for (int ch = 0; ch < 4; ++ch) {
+        const Real m = rmul(v[ch], w[ax]);
+        v[ch] = radd(m, __shfl_xor_sync(kFull, m, 4 >> ax));
+      }
     }
+    if (in && corner < 4) out[4 * i + corner] = pick4(v, corner);
   }
 }
 
+// A thread per corner, as trilinear_gather_kernel (768,000 samples 95 us, now 54).
 template <typename Real, typename Store>
 __global__ void trilinear_scatter_kernel(GridP<Real> g, const Real* __restrict__ n,
-                                         const int64_t* __restrict__ corners, int64_t count,
+                                         const int64_t* __restrict__ corners, int64_t lanes,
                                          const Real* __restrict__ dout, Real* __restrict__ grad,
                                          int* __restrict__ status) {
-  PGB_FOR(i, count) {
-    const Real wx = frac_ref(n[3 * i]), wy = frac_ref(n[3 * i + 1]), wz = frac_ref(n[3 * i + 2]);
-    const Real ux = rsub(Real(1), wx), uy = rsub(Real(1), wy), uz = rsub(Real(1), wz);
-    Real dv[4];
+  PGB_FOR(t, lanes) {
+    const int64_t i = t >> 3;
+    const int corner = (int)t & 7;
+    uint64_t c;
+    if (!corner_cell(g, corners + 3 * t, c, status)) continue;
+    Real w[3];
 #pragma unroll
-    for (int ch = 0; ch < 4; ++ch) dv[ch] = dout[4 * i + ch];
-#pragma unroll
-    for (int corner = 0; corner < 8; ++corner) {
-      const Real sz = (corner & 1) ? uz : wz;
-      const Real sy = (corner & 2) ? uy : wy;
-      const Real sx = (corner & 4) ? ux : wx;
-      uint64_t c;
-      if (!corner_cell(g, corners + 24 * i + 3 * corner, c, status)) continue;
-      Real cv[4];
-      if (g.clip) CellIO<Store>::load(g.cells, c, cv);
-      Real gv[4];
-      bool any = false;
-#pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        gv[ch] = rmul(rmul(rmul(dv[ch], sz), sy), sx);
-        if (g.clip && !in01(cv[ch])) gv[ch] = Real(0);
-        any |= gv[ch] != Real(0);
-      }
-      if (any) grad_add(grad, c, gv);
+    for (int ax = 0; ax < 3; ++ax) {
+      const Real f = frac_ref(__ldg(n + 3 * i + ax));
+      w[ax] = (corner & (4 >> ax)) ? rsub(Real(1), f) : f;
     }
+    Real cv[4], gv[4];
+    if (g.clip) CellIO<Store>::load(g.cells, c, cv);
+    bool any = false;
+#pragma unroll
+    for (int ch = 0; ch < 4; ++ch) {
+      gv[ch] = rmul(rmul(rmul(__ldg(dout + 4 * i + ch), w[2]), w[1]), w[0]);
+      if (g.clip && !in01(cv[ch])) gv[ch] = Real(0);
+      any |= gv[ch] != Real(0);
+    }
+    if (any) grad_add(grad, c, gv);
   }
 }
 
@@ -630,7 +684,9 @@ int op_coords_min(const float* coords, int64_t count, float* out, cudaStream_t s
 
 int op_normalize(const float* samples, int64_t count, const float* gmin, float pd, float* out,
                  cudaStream_t s) {
-  normalize_kernel<<<blocks_for(count), kThreads, 0, s>>>(samples, count, gmin, pd, out);
+  const int64_t fours = (((uintptr_t)samples | (uintptr_t)out) & 15u) == 0 ? count / 4 : 0;
+  normalize_kernel<<<blocks_for(std::max(fours, count - 4 * fours)), kThreads, 0, s>>>(samples, count, fours,
+                                                                                      gmin, pd, out);
   return after_launch();
 }
 
@@ -651,16 +707,16 @@ static int nearest_scatter_t(const GridP<Real>& g, const void* n, int64_t count,
 template <typename Real, typename Store>
 static int trilinear_gather_t(const GridP<Real>& g, const void* n, const int64_t* corners,
                               int64_t count, void* out, int* status, cudaStream_t s) {
-  trilinear_gather_kernel<Real, Store><<<blocks_for(count), kThreads, 0, s>>>(
-      g, (const Real*)n, corners, count, (Real*)out, status);
+  trilinear_gather_kernel<Real, Store><<<blocks_for(8 * count), kThreads, 0, s>>>(
+      g, (const Real*)n, corners, 8 * count, (Real*)out, status);
   return after_launch();
 }
 template <typename Real, typename Store>
 static int trilinear_scatter_t(const GridP<Real>& g, const void* n, const int64_t* corners,
                                int64_t count, const void* dout, void* grad, int* status,
                                cudaStream_t s) {
-  trilinear_scatter_kernel<Real, Store><<<blocks_for(count), kThreads, 0, s>>>(
-      g, (const Real*)n, corners, count, (const Real*)dout, (Real*)grad, status);
+  trilinear_scatter_kernel<Real, Store><<<blocks_for(8 * count), kThreads, 0, s>>>(
+      g, (const Real*)n, corners, 8 * count, (const Real*)dout, (Real*)grad, status);
   return after_launch();
 }
 
@@ -741,10 +797,16 @@ int op_scatter_cells_f64(const GridP<double>& g, const int64_t* idx, int64_t cou
   return scatter_cells_t<double, double>(g, idx, count, dv, grad, status, s);
 }
 
-int op_corner_indices(const void* n, int f64, int64_t count, int64_t* out, cudaStream_t s) {
-  if (f64) corner_indices_kernel<double><<<blocks_for(count), kThreads, 0, s>>>((const double*)n, count, out);
-  else corner_indices_kernel<float><<<blocks_for(count), kThreads, 0, s>>>((const float*)n, count, out);
+template <typename Real>
+static int corner_indices_t(const Real* n, int64_t count, int64_t* out, cudaStream_t s) {
+  if (((uintptr_t)out & 15u) == 0)
+    corner_indices_kernel<Real, 2><<<blocks_for(12 * count), kThreads, 0, s>>>(n, 12 * count, out);
+  else
+    corner_indices_kernel<Real, 1><<<blocks_for(24 * count), kThreads, 0, s>>>(n, 24 * count, out);
   return after_launch();
+}
+int op_corner_indices(const void* n, int f64, int64_t count, int64_t* out, cudaStream_t s) {
+  return f64 ? corner_indices_t((const double*)n, count, out, s) : corner_indices_t((const float*)n, count, out, s);
 }
 
 int op_in_bounds(const void* idx, int kind, int64_t count, const int dims[3], uint8_t* out,
@@ -760,7 +822,16 @@ int op_in_bounds(const void* idx, int kind, int64_t count, const int dims[3], ui
 }
 
 int op_wrap(int64_t* idx, int64_t count, const int dims[3], cudaStream_t s) {
-  wrap_kernel<<<blocks_for(count), kThreads, 0, s>>>(idx, count, dims[0], dims[1], dims[2]);
+  const int64_t total = 3 * count;
+  const int64_t pairs = ((uintptr_t)idx & 15u) == 0 ? total / 2 : 0;
+  if (pairs > 0) {
+    wrap_pairs_kernel<<<blocks_for(pairs), kThreads, 0, s>>>(reinterpret_cast<longlong2*>(idx), pairs,
+                                                             dims[0], dims[1], dims[2]);
+    const int st = after_launch();
+    if (st || 2 * pairs == total) return st;
+  }
+  wrap_kernel<<<blocks_for(total - 2 * pairs), kThreads, 0, s>>>(idx, 2 * pairs, total, dims[0], dims[1],
+                                                                 dims[2]);
   return after_launch();
 }
 

@@ -50,8 +50,17 @@ template <typename Real>
 __device__ __forceinline__ bool in01(Real x) { return x >= Real(0) && x <= Real(1); }
 
 // Python-style floor modulo for a positive modulus (src/grid_functions.py:75-77).
+// Most indices are in range or a little outside it; a 64-bit remainder is a hundred
+// instructions.
 __device__ __forceinline__ long long floor_mod(long long a, long long m) {
-  long long r = a % m;
+  if ((unsigned long long)a < (unsigned long long)m) return a;
+  const long long near = a < 0 ? a + m : a - m;
+  if ((unsigned long long)near < (unsigned long long)m) return near;
+  if (a == (int)a && m == (int)m) {
+    const int r = (int)a % (int)m;
+    return r < 0 ? r + m : r;
+  }
+  const long long r = a % m;
   return r < 0 ? r + m : r;
 }
 
