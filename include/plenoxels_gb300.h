@@ -264,6 +264,11 @@ int pgb_adam_tv_step(const float* param_in, float* param_out, float* grad, float
                      const double* tv_sumsq, float tv_weight, double lr, double beta1, double beta2,
                      double eps, int64_t step, int32_t zero_grad, pgb_stream_t stream);
 
+/* The three losses of a training step (scripts/train.py:156-177) in one place: [weighted MSE, TV
+ * term, beta term] from the render step's losses and pgb_tv_sumsq's result (NULL: no TV term). */
+int pgb_step_losses(const float* step_losses, const double* tv_sumsq, double tv_weight, int32_t with_beta,
+                    float* losses_out, pgb_stream_t stream);
+
 /* src/grid_functions.py:173-181 average_pool3d_grid (scripts/train.py:108-123): average of
  * a cubic window of `window` cells, stride `stride`, no padding, of a contiguous fp32
  * [X,Y,Z,4] grid into [Xo,Yo,Zo,4], Xo = (X - window) / stride + 1. pgb_avg_pool3d_shape

@@ -105,6 +105,7 @@ _SIGNATURES = {
     "pgb_batch_workspace_bytes": (c_int64, [c_int64]),
     "pgb_batch_train": (c_int32, [_P, c_int32, c_int32, c_int32, c_int32, _P, _P, _P, _P, c_int64, c_float,
                                   c_int32, c_uint64, c_double, _P, _P, _P, c_int32, c_int32, c_int32, _P]),
+    "pgb_step_losses": (c_int32, [_P, _P, c_double, c_int32, _P, _P]),
     "pgb_tv_workspace_bytes": (c_int64, []),
     "pgb_tv_sumsq": (c_int32, [_P, POINTER(c_int32), _P, _P, _P]),
     "pgb_tv_grad": (c_int32, [_P, POINTER(c_int32), _P, c_float, _P, _P]),
@@ -186,18 +187,22 @@ def check(status: int, what: str) -> None:
 
 
 def stream_of(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    """The current stream of t's device, as the raw handle (without a Stream object)."""
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
 
 
 def require_cuda(*tensors: torch.Tensor) -> None:
+    first = None
     for t in tensors:
         if not isinstance(t, torch.Tensor):
             raise TypeError(f"expected a torch.Tensor, got {type(t).__name__}")
         if not t.is_cuda:
             raise ValueError("plenoxels_gb300 operators take CUDA tensors (there is no CPU path)")
-    devs = {t.device for t in tensors}
-    if len(devs) > 1:
-        raise ValueError(f"tensors are on different devices: {sorted(map(str, devs))}")
+        if first is None:
+            first = t.get_device()
+        elif t.get_device() != first:
+            devs = {str(x.device) for x in tensors}
+            raise ValueError(f"tensors are on different devices: {sorted(devs)}")
 
 
 def ptr(t: torch.Tensor | None) -> int | None:
@@ -220,17 +225,10 @@ def make_grid(cells: torch.Tensor, origin, points_distance: float, mode: int, cl
         raise TypeError(f"grid dtype {cells.dtype} not supported (float32, bfloat16, float64)")
     if not cells.is_contiguous():
         raise ValueError("grid must be contiguous channels-last [X,Y,Z,4]")
-    g = PgbGrid()
-    g.cells = cells.data_ptr()
-    g.dtype = STORAGE_CODES[cells.dtype]
-    g.dims[0], g.dims[1], g.dims[2] = (int(s) for s in cells.shape[:3])
-    for a in range(3):
-        g.origin[a] = float(origin[a])
-    g.points_distance = float(points_distance)
-    g.clip = 1 if clip else 0
-    g.mode = mode
-    g.alpha_floor = float(alpha_floor)
-    return g
+    x, y, z, _ = cells.shape
+    return PgbGrid(cells.data_ptr(), STORAGE_CODES[cells.dtype], (x, y, z),
+                   (float(origin[0]), float(origin[1]), float(origin[2])), float(points_distance),
+                   1 if clip else 0, mode, float(alpha_floor))
 
 
 def dims3(shape) -> ctypes.Array:

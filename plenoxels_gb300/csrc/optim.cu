@@ -223,6 +223,13 @@ __global__ void __launch_bounds__(kTvThreads, 5) adam_tv_kernel(
   }
 }
 
+__global__ void step_losses_kernel(const float* __restrict__ step, const double* __restrict__ tv_sumsq,
+                                   double tv_weight, int with_beta, float* __restrict__ out) {
+  out[0] = step[0];
+  out[1] = tv_sumsq != nullptr ? (float)(tv_weight * sqrt(tv_sumsq[0])) : 0.f;
+  out[2] = with_beta ? step[1] : 0.f;
+}
+
 inline unsigned stream_blocks(int64_t n) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 152 * 48));
 }
@@ -303,6 +310,13 @@ int pgb_adam_tv_step(const float* param_in, float* param_out, float* grad, float
       reinterpret_cast<float4*>(grad), reinterpret_cast<float4*>(exp_avg),
       reinterpret_cast<float4*>(exp_avg_sq), reinterpret_cast<float4*>(abs_grad_accum), dims[0],
       dims[1], dims[2], tv_sumsq, tv_weight, k, zero_grad ? 1 : 0);
+  return after_launch();
+}
+
+int pgb_step_losses(const float* step_losses, const double* tv_sumsq, double tv_weight, int32_t with_beta,
+                    float* losses_out, pgb_stream_t stream) {
+  if (!step_losses || !losses_out) return PGB_ERR_ARG;
+  step_losses_kernel<<<1, 1, 0, stream>>>(step_losses, tv_sumsq, tv_weight, with_beta, losses_out);
   return after_launch();
 }
 

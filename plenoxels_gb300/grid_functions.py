@@ -53,8 +53,10 @@ def grid_origin(shape, points_distance: float, dtype=torch.float32):
     if dtype == torch.float64:
         return tuple(float(np.float64(1 - math.ceil(s / 2)) * np.float64(points_distance))
                      for s in shape[:3])
-    return tuple(float(np.float32(1 - math.ceil(s / 2)) * np.float32(points_distance))
-                 for s in shape[:3])
+    # a product of two fp32 numbers is exact in double: one rounding each, as fp32 arithmetic's
+    f32 = ctypes.c_float
+    pd = f32(points_distance).value
+    return tuple(f32(f32(1 - math.ceil(s / 2)).value * pd).value for s in shape[:3])
 
 
 def _grid_desc(grid, mode, clip=False):

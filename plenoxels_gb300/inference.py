@@ -17,10 +17,10 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import check, ptr, require_cuda
+from ._lib import check, ptr, require_cuda, stream_of
 from .grid_functions import grid_origin
-from .ray_sampling import generate_rays_batched
-from .render import _rays_desc
+from .ray_sampling import _f32, generate_rays_batched
+from .render import _check_rays, _rays_desc, _render_cfg, _render_forward
 
 PARAM_KEYS = ("device", "number_of_rays", "num_samples", "delta_step", "even_spread",
               "camera_ray", "points_distance", "gridsize")
@@ -92,7 +92,6 @@ def render_camera_images(grid, transforms, height, width, camera_angle_x, near, 
     require_cuda(grid, transforms)
     if height != width:
         raise ValueError("render_camera_images renders square images")
-    from .render import render_rays
     dev = grid.device
     C, H, W = transforms.shape[0], int(height), int(width)
     rows = torch.arange(H, device=dev, dtype=torch.float32)
@@ -101,11 +100,19 @@ def render_camera_images(grid, transforms, height, width, camera_angle_x, near, 
     blank = torch.zeros(1, H, W, 4, device=dev)
     out = torch.empty(C, H, W, 4, dtype=torch.float32, device=dev)
     g = grid.detach().contiguous()
+    if grid_min is None:
+        grid_min = grid_origin(g.shape, points_distance, _lib.real_dtype(g.dtype))
+    cfg = _render_cfg(grid_min, points_distance, mode, delta_step, num_samples, stratified=stratified,
+                      seed=seed)
+    lib, R = _lib.load(), H * W
+    dirs = torch.empty(R, 3, dtype=torch.float32, device=dev)
+    pixels = torch.empty(R, 4, dtype=torch.float32, device=dev)
     for c in range(C):
-        T = transforms[c:c + 1].contiguous()
-        dirs, _ = generate_rays_batched(blank, H * W, T, camera_angle_x, device=dev, ray_uv=uv)
+        T = _f32(transforms[c:c + 1], "render_camera_images")
+        # the uniforms are pixel centres, inside the images by construction: no status word
+        check(lib.pgb_generate_rays(ptr(T), 1, R, float(camera_angle_x), ptr(blank), H, W, ptr(uv), 0, ptr(dirs),
+                                    ptr(pixels), None, stream_of(T)), "render_camera_images")
         origins = (T[0, :3, 3] + near * dirs).contiguous()
-        rgba = render_rays(g, origins, dirs, delta_step, num_samples, points_distance, grid_min,
-                           mode=mode, stratified=stratified, seed=seed)
-        out[c] = rgba.reshape(H, W, 4)
+        _check_rays(g, origins, dirs)
+        _render_forward(g, origins, dirs, cfg, out[c])
     return out

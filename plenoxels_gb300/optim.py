@@ -7,7 +7,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib
-from ._lib import check, ptr, require_cuda
+from ._lib import check, ptr, require_cuda, stream_of
 
 
 class FusedAdam:
@@ -33,17 +33,20 @@ class FusedAdam:
         self._tv_ws = torch.zeros(lib.pgb_tv_workspace_bytes(), dtype=torch.uint8, device=grid.device)
         self.tv_sumsq = torch.zeros((), dtype=torch.float64, device=grid.device)
 
-    def add_tv(self, grad, weight, grid=None):
-        """Adds the gradient of weight * tv_loss(grid) (scripts/train.py:163-165) to grad;
-        returns the term's value as a device scalar. grid defaults to the optimised grid
-        (the pooled grid while progressive growing runs)."""
-        grid = self.grid if grid is None else grid
+    def _tv_pass(self, grad, weight, grid):
+        """add_tv without its value: self.tv_sumsq holds the squared norm."""
         lib = _lib.load()
-        s = torch.cuda.current_stream(grid.device).cuda_stream
+        s = stream_of(grid)
         dims = _lib.dims3(grid.shape)
         check(lib.pgb_tv_sumsq(ptr(grid), dims, ptr(self.tv_sumsq), ptr(self._tv_ws), s), "tv loss")
         check(lib.pgb_tv_grad(ptr(grid), dims, ptr(self.tv_sumsq), float(weight), ptr(grad), s),
               "tv loss")
+
+    def add_tv(self, grad, weight, grid=None):
+        """Adds the gradient of weight * tv_loss(grid) (scripts/train.py:163-165) to grad;
+        returns the term's value as a device scalar. grid defaults to the optimised grid
+        (the pooled grid while progressive growing runs)."""
+        self._tv_pass(grad, weight, self.grid if grid is None else grid)
         return float(weight) * self.tv_sumsq.sqrt()
 
     @torch.no_grad()
@@ -52,7 +55,7 @@ class FusedAdam:
         if grad is None or grad.shape != self.grid.shape or grad.dtype != torch.float32:
             raise ValueError("step needs the grid's float32 gradient")
         self.step_count += 1
-        s = torch.cuda.current_stream(self.grid.device).cuda_stream
+        s = stream_of(self.grid)
         check(_lib.load().pgb_adam_step(ptr(self.grid), ptr(grad), ptr(self.exp_avg),
                                         ptr(self.exp_avg_sq), ptr(self.abs_grad), self.grid.numel(),
                                         self.lr, self.betas[0], self.betas[1], self.eps,
@@ -65,7 +68,7 @@ class FusedAdam:
         the full gradient in memory. scratch: the bytes of grid_functions.pool_shape."""
         g = self.grid
         self.step_count += 1
-        s = torch.cuda.current_stream(g.device).cuda_stream
+        s = stream_of(g)
         check(_lib.load().pgb_avg_pool3d_bwd_adam(
             ptr(pooled_grad), _lib.dims3(g.shape), window, stride, ptr(scratch), ptr(g), ptr(self.exp_avg),
             ptr(self.exp_avg_sq), ptr(self.abs_grad), self.lr, self.betas[0], self.betas[1], self.eps,
@@ -80,13 +83,18 @@ class FusedAdam:
         read while cells are updated), which becomes ``self.grid``; the previous grid
         tensor is left holding the pre-step values. Returns weight * tv_loss as a device
         scalar."""
+        self._step_tv_pass(grad, weight, out, zero_grad)
+        return float(weight) * self.tv_sumsq.sqrt()
+
+    def _step_tv_pass(self, grad, weight, out, zero_grad=True):
+        """step_tv without its value: self.tv_sumsq holds the squared norm."""
         g = self.grid
         if out.shape != g.shape or out.dtype != g.dtype or not out.is_contiguous() or out.data_ptr() == g.data_ptr():
             raise ValueError("out must be a separate contiguous float32 buffer of the grid's shape")
         if grad is None or grad.shape != g.shape or grad.dtype != torch.float32:
             raise ValueError("step_tv needs the grid's float32 gradient")
         lib = _lib.load()
-        s = torch.cuda.current_stream(g.device).cuda_stream
+        s = stream_of(g)
         dims = _lib.dims3(g.shape)
         check(lib.pgb_tv_sumsq(ptr(g), dims, ptr(self.tv_sumsq), ptr(self._tv_ws), s), "tv loss")
         self.step_count += 1
@@ -95,4 +103,3 @@ class FusedAdam:
                                    self.betas[0], self.betas[1], self.eps, self.step_count,
                                    1 if zero_grad else 0, s), "adam + tv step")
         self.grid = out
-        return float(weight) * self.tv_sumsq.sqrt()

@@ -35,27 +35,19 @@ def _transmittance(name: str) -> int:
     return TRANSMITTANCE[name]
 
 
+_NO_BACKGROUND = (0.0, 0.0, 0.0)
+
+
 def _rays_desc(origins, dirs, num_rays, num_samples, delta_step, stratified, seed, term_threshold,
                cameras=None, background=None, log_t=0, chunk_samples=0, first_ray=0,
                grad_marks=None) -> PgbRays:
-    r = PgbRays()
-    r.origins = ptr(origins)
-    r.dirs = ptr(dirs)
-    r.cameras = ctypes.pointer(cameras) if cameras is not None else None
-    r.num_rays = int(num_rays)
-    r.num_samples = int(num_samples)
-    r.delta_step = float(delta_step)
-    r.stratified = 1 if stratified else 0
-    r.seed = int(seed) & 0xFFFFFFFFFFFFFFFF
-    r.term_threshold = float(term_threshold)
-    if background is not None:
-        r.use_background = 1
-        r.background[:] = [float(v) for v in background]
-    r.log_transmittance = int(log_t)
-    r.chunk_samples = int(chunk_samples)
-    r.first_ray = int(first_ray)
-    r.grad_marks = ptr(grad_marks)
-    return r
+    if background is not None and len(background) != 3:
+        raise ValueError("background must have 3 values")
+    return PgbRays(ptr(origins), ptr(dirs), ctypes.pointer(cameras) if cameras is not None else None,
+                   int(num_rays), int(num_samples), float(delta_step), 1 if stratified else 0,
+                   int(seed) & 0xFFFFFFFFFFFFFFFF, float(term_threshold), 0 if background is None else 1,
+                   _NO_BACKGROUND if background is None else tuple(float(v) for v in background),
+                   int(log_t), int(chunk_samples), int(first_ray), ptr(grad_marks))
 
 
 def _check_rays(grid, origins, dirs):
@@ -69,18 +61,45 @@ def _check_rays(grid, origins, dirs):
         raise ValueError("origins and dirs must have the same number of rays")
 
 
+def _render_cfg(grid_min, points_distance, mode, delta_step, num_samples, clip=True, stratified=False, seed=0,
+                term_threshold=0.0, background=None, transmittance="product", chunk_samples=0):
+    return dict(origin=tuple(float(x) for x in grid_min), points_distance=float(points_distance),
+                mode=_mode(mode), clip=bool(clip), num_samples=int(num_samples),
+                delta_step=float(delta_step), stratified=bool(stratified), seed=int(seed),
+                term_threshold=float(term_threshold),
+                background=None if background is None else tuple(float(v) for v in background),
+                log_t=_transmittance(transmittance), chunk_samples=int(chunk_samples))
+
+
+def _render_descs(grid, origins, dirs, cfg):
+    return (_lib.make_grid(grid, cfg["origin"], cfg["points_distance"], cfg["mode"], cfg["clip"]),
+            _rays_desc(origins, dirs, origins.shape[0], cfg["num_samples"], cfg["delta_step"],
+                       cfg["stratified"], cfg["seed"], cfg["term_threshold"],
+                       background=cfg["background"], log_t=cfg["log_t"],
+                       chunk_samples=cfg["chunk_samples"]))
+
+
+def _render_forward(grid, origins, dirs, cfg, rgba=None):
+    """The forward launch; rgba: a contiguous [R,4] tensor to write to."""
+    if rgba is None:
+        rgba = torch.empty(origins.shape[0], 4, dtype=_lib.real_dtype(grid.dtype), device=grid.device)
+    gdesc, rdesc = _render_descs(grid, origins, dirs, cfg)
+    check(_lib.load().pgb_render_fwd(gdesc, rdesc, rgba.data_ptr(), stream_of(grid)), "render_rays")
+    return rgba
+
+
+def _wants_autograd(*tensors):
+    """Whether a call has to go through its autograd Function: a gradient may be asked for,
+    or a transform (vmap, forward-mode, functional tracing) is at work and decides itself."""
+    if torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0:
+        return True
+    return torch.is_grad_enabled() and any(t.requires_grad for t in tensors)
+
+
 class _RenderRays(torch.autograd.Function):
     @staticmethod
     def forward(ctx, grid, origins, dirs, cfg):
-        lib = _lib.load()
-        R = origins.shape[0]
-        rgba = torch.empty(R, 4, dtype=_lib.real_dtype(grid.dtype), device=grid.device)
-        gdesc = _lib.make_grid(grid, cfg["origin"], cfg["points_distance"], cfg["mode"], cfg["clip"])
-        rdesc = _rays_desc(origins, dirs, R, cfg["num_samples"], cfg["delta_step"],
-                           cfg["stratified"], cfg["seed"], cfg["term_threshold"],
-                           background=cfg["background"], log_t=cfg["log_t"],
-                           chunk_samples=cfg["chunk_samples"])
-        check(lib.pgb_render_fwd(gdesc, rdesc, ptr(rgba), stream_of(grid)), "render_rays")
+        rgba = _render_forward(grid, origins, dirs, cfg)
         ctx.save_for_backward(grid, origins, dirs)
         ctx.cfg = cfg
         return rgba
@@ -88,18 +107,16 @@ class _RenderRays(torch.autograd.Function):
     @staticmethod
     def backward(ctx, d_rgba):
         grid, origins, dirs = ctx.saved_tensors
-        cfg = ctx.cfg
         lib = _lib.load()
         s = stream_of(grid)
         grad = torch.empty(grid.shape, dtype=_lib.real_dtype(grid.dtype), device=grid.device)
-        check(lib.pgb_fill_zero(ptr(grad), grad.numel() * grad.element_size(), s), "backward")
-        d_rgba = d_rgba.to(grad.dtype).contiguous()
-        gdesc = _lib.make_grid(grid, cfg["origin"], cfg["points_distance"], cfg["mode"], cfg["clip"])
-        rdesc = _rays_desc(origins, dirs, origins.shape[0], cfg["num_samples"], cfg["delta_step"],
-                           cfg["stratified"], cfg["seed"], cfg["term_threshold"],
-                           background=cfg["background"], log_t=cfg["log_t"],
-                           chunk_samples=cfg["chunk_samples"])
-        check(lib.pgb_render_bwd(gdesc, rdesc, ptr(d_rgba), ptr(grad), s), "render_rays backward")
+        check(lib.pgb_fill_zero(grad.data_ptr(), grad.numel() * grad.element_size(), s), "backward")
+        if d_rgba.dtype != grad.dtype:
+            d_rgba = d_rgba.to(grad.dtype)
+        d_rgba = d_rgba.contiguous()
+        gdesc, rdesc = _render_descs(grid, origins, dirs, ctx.cfg)
+        check(lib.pgb_render_bwd(gdesc, rdesc, d_rgba.data_ptr(), grad.data_ptr(), s),
+              "render_rays backward")
         return grad, None, None, None
 
 
@@ -120,13 +137,12 @@ def render_rays(grid, origins, dirs, delta_step, num_samples, points_distance, g
     _check_rays(grid, origins, dirs)
     if grid_min is None:
         grid_min = grid_origin(grid.shape, points_distance, _lib.real_dtype(grid.dtype))
-    cfg = dict(origin=tuple(float(x) for x in grid_min), points_distance=float(points_distance),
-               mode=_mode(mode), clip=bool(clip), num_samples=int(num_samples),
-               delta_step=float(delta_step), stratified=bool(stratified), seed=int(seed),
-               term_threshold=float(term_threshold),
-               background=None if background is None else tuple(float(v) for v in background),
-               log_t=_transmittance(transmittance), chunk_samples=int(chunk_samples))
-    return _RenderRays.apply(grid.contiguous(), origins.contiguous(), dirs.contiguous(), cfg)
+    cfg = _render_cfg(grid_min, points_distance, mode, delta_step, num_samples, clip, stratified, seed,
+                      term_threshold, background, transmittance, chunk_samples)
+    grid, origins, dirs = grid.contiguous(), origins.contiguous(), dirs.contiguous()
+    if not _wants_autograd(grid, origins, dirs):
+        return _render_forward(grid, origins, dirs, cfg)
+    return _RenderRays.apply(grid, origins, dirs, cfg)
 
 
 def render_sample_indices(grid, origins, dirs, delta_step, num_samples, points_distance,
@@ -279,25 +295,24 @@ class FusedTrainStep:
         buf = self._grads[b]
         lib = _lib.load()
         if self._marks is None:
-            check(lib.pgb_fill_zero(ptr(buf), buf.numel() * buf.element_size(), stream.cuda_stream),
-                  "train step")
+            check(lib.pgb_fill_zero(ptr(buf), buf.numel() * buf.element_size(), stream), "train step")
         else:
             check(lib.pgb_clear_marked(ptr(buf), 4 * buf.element_size(), buf.numel() // 4,
-                                       ptr(self._marks[b]), stream.cuda_stream), "train step")
+                                       ptr(self._marks[b]), stream), "train step")
 
     def _gradient_for_step(self, zero_grad):
-        main = torch.cuda.current_stream(self.grid.device)
         if not zero_grad:
             return self.grad
         if self._side is None:
-            self._fill(0, main)
+            self._fill(0, stream_of(self.grid))
             self._buf = 0
             return self.grad
+        main = torch.cuda.current_stream(self.grid.device)
         b = self._cur
         buf = self._grads[b]
         self._buf = b
         if self._zeroed[b] is None:
-            self._fill(b, main)
+            self._fill(b, main.cuda_stream)
         else:
             main.wait_event(self._zeroed[b])
         # zero the other buffer for the next step, after everything already queued on the
@@ -306,7 +321,7 @@ class FusedTrainStep:
         ready = torch.cuda.Event()
         ready.record(main)
         self._side.wait_event(ready)
-        self._fill(o, self._side)
+        self._fill(o, self._side.cuda_stream)
         done = torch.cuda.Event()
         done.record(self._side)
         self._zeroed[o] = done
@@ -336,23 +351,24 @@ class FusedTrainStep:
         grad = self._gradient_for_step(zero_grad)
         if self._marks is not None:
             rdesc.grad_marks = ptr(self._marks[self._buf])
-        stream = torch.cuda.current_stream(self.grid.device)
+        stream = stream_of(self.grid)
         gdesc = _lib.make_grid(self.grid, self.grid_min, self.points_distance, self.mode, self.clip)
         ev = None
         if self.kernel_events is not None:
+            main = torch.cuda.current_stream(self.grid.device)
             ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
-            ev[0].record(stream)
+            ev[0].record(main)
         if self.beta == 0.0:
             check(lib.pgb_render_train(gdesc, rdesc, ptr(target), self.loss_weight, ptr(rgba_out),
-                                       ptr(grad), ptr(losses), ptr(self.workspace),
-                                       stream.cuda_stream), "train step")
+                                       ptr(grad), ptr(losses), ptr(self.workspace), stream),
+                  "train step")
         else:
             terms = _lib.PgbLossTerms(self.loss_weight, self.beta, self.beta_eps)
             check(lib.pgb_render_train_terms(gdesc, rdesc, ptr(target), terms, ptr(rgba_out),
-                                             ptr(grad), ptr(losses), ptr(self.workspace),
-                                             stream.cuda_stream), "train step")
+                                             ptr(grad), ptr(losses), ptr(self.workspace), stream),
+                  "train step")
         if ev is not None:
-            ev[1].record(stream)
+            ev[1].record(main)
             self.kernel_events.append(ev)
         return self.loss if loss_out is None else loss_out[0]
 

@@ -24,7 +24,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import check, ptr
+from ._lib import check, ptr, stream_of
 from .grid_functions import pool_shape
 from .optim import FusedAdam
 from .render import FusedTrainStep
@@ -79,7 +79,7 @@ class Trainer:
     def _run(self, launch):
         r = self.field(self.step_index) if self.progressive else 0
         lib = _lib.load()
-        s = torch.cuda.current_stream(self.grid.device).cuda_stream
+        s = stream_of(self.grid)
         full_grad = self.render.grad
         if r > 1:
             pooled, step, stride, scratch = self._pooled_step(r)
@@ -92,22 +92,19 @@ class Trainer:
             # the Adam pass left the gradient zeroed: accumulate into it directly
             launch(self.render, False)
             render_step, tv_grid, tv_grad = self.render, self.grid, full_grad
-        self.losses[0] = render_step.losses[0]
-        self.losses[2] = render_step.losses[1] if self.beta != 0.0 else 0.0
-        self.losses[1] = 0.0
         if self.tv > 0.0 and r < 19 and self.fuse_tv and r <= 1:
             # TV on the full grid: its gradient is evaluated inside the Adam pass, which
             # writes the new grid to the spare buffer; the buffers then swap roles
             if self._spare is None:
                 self._spare = torch.empty_like(self.grid)
             old = self.grid
-            self.losses[1] = self.opt.step_tv(full_grad, self.tv, self._spare)
+            self.opt._step_tv_pass(full_grad, self.tv, self._spare)
             self.grid, self._spare = self._spare, old
             self.render.grid = self.grid
-            self.step_index += 1
-            return self.losses
-        if self.tv > 0.0 and r < 19:
-            self.losses[1] = self.opt.add_tv(tv_grad, self.tv, grid=tv_grid)
+            return self._finish(render_step, True, s)
+        with_tv = self.tv > 0.0 and r < 19
+        if with_tv:
+            self.opt._tv_pass(tv_grad, self.tv, tv_grid)
         if r > 1 and full_grad._version == self._grad_version:
             self.opt.step_pooled(render_step.grad, r, stride, scratch)
         else:
@@ -116,6 +113,14 @@ class Trainer:
                                              stride, ptr(scratch), ptr(full_grad), s), "pooled grid")
                 self._grad_version = full_grad._version
             self.opt.step(full_grad)
+        return self._finish(render_step, with_tv, s)
+
+    def _finish(self, render_step, with_tv, s):
+        """The step's three losses in one small launch (assigning a Python number to a GPU
+        tensor's element copies it from pageable memory, which waits for the stream)."""
+        check(_lib.load().pgb_step_losses(ptr(render_step.losses), ptr(self.opt.tv_sumsq) if with_tv else None,
+                                          self.tv, 1 if self.beta != 0.0 else 0, ptr(self.losses), s),
+              "train step")
         self.step_index += 1
         return self.losses
 
