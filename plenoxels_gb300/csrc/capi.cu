@@ -54,8 +54,15 @@ template <typename Real>
 int render_common(const pgb_grid* g, const pgb_rays* r, int phase, void* rgba_out,
                   const void* d_rgba, const void* target, double loss_w, void* grad,
                   void* loss_out, void* workspace, cudaStream_t s, double beta_w = 0.0,
-                  float beta_eps = 0.f) {
+                  float beta_eps = 0.f, void* clear_grad = nullptr, uint32_t* clear_marks = nullptr) {
   RenderArgs<Real> a = render_args<Real>(g, r);
+  if (clear_grad) {
+    const int64_t cells = (int64_t)g->dims[0] * g->dims[1] * g->dims[2];
+    a.clear_grad = (uint4*)clear_grad;
+    a.clear_total16 = cells;  // fp32: 16 bytes a cell
+    a.clear_marks = clear_marks;
+    a.clear_words = mark_words(cells);
+  }
   a.beta_w = beta_w;
   a.beta_eps = beta_eps;
   const double samples = (double)r->num_rays * (double)r->num_samples;
@@ -150,6 +157,36 @@ int pgb_render_train_terms(const pgb_grid* grid, const pgb_rays* rays, const voi
   return render_common<float>(grid, rays, kTrain, rgba_out, nullptr, target, terms->mse_weight,
                               grad_cells, losses_out, workspace, stream, terms->beta_weight,
                               terms->beta_eps);
+}
+
+int pgb_render_train_clear(const pgb_grid* grid, const pgb_rays* rays, const void* target,
+                           const pgb_loss_terms* terms, void* rgba_out, void* grad_cells,
+                           void* losses_out, void* workspace, void* clear_grad_cells,
+                           uint32_t* clear_grad_marks, pgb_stream_t stream) {
+  if (!terms) return PGB_ERR_ARG;
+  int st = check_grid(grid);
+  if (st) return st;
+  if ((st = check_rays(grid, rays, true))) return st;
+  if (!grad_cells || !losses_out || !workspace || !clear_grad_cells) return PGB_ERR_ARG;
+  if (!rays->cameras && rays->num_rays > 0 && !target) return PGB_ERR_ARG;
+  // the kernel writes one buffer while it clears the other
+  if (clear_grad_cells == grad_cells || (clear_grad_marks && clear_grad_marks == rays->grad_marks))
+    return PGB_ERR_ARG;
+  if (!aligned(grad_cells, 16) || !aligned(workspace, 16) || !aligned(clear_grad_cells, 16) ||
+      !aligned(clear_grad_marks, 4))
+    return PGB_ERR_ALIGN;
+  if (grid->dtype == PGB_F64) {  // fp64 launches keep a clear of their own
+    const int64_t cells = (int64_t)grid->dims[0] * grid->dims[1] * grid->dims[2];
+    st = clear_grad_marks ? op_clear_marked(clear_grad_cells, 32, cells, clear_grad_marks, stream)
+                          : op_fill_zero(clear_grad_cells, 32 * cells, stream);
+    if (st) return st;
+    return render_common<double>(grid, rays, kTrain, rgba_out, nullptr, target, terms->mse_weight,
+                                 grad_cells, losses_out, workspace, stream, terms->beta_weight,
+                                 terms->beta_eps);
+  }
+  return render_common<float>(grid, rays, kTrain, rgba_out, nullptr, target, terms->mse_weight,
+                              grad_cells, losses_out, workspace, stream, terms->beta_weight,
+                              terms->beta_eps, clear_grad_cells, clear_grad_marks);
 }
 
 int pgb_render_sample_indices(const pgb_grid* grid, const pgb_rays* rays, int64_t* index_out,

@@ -252,7 +252,8 @@ __device__ __forceinline__ uint64_t mark_unit_of(uint64_t cell) { return cell >>
 // warp takes 32 consecutive words per round (one coalesced load, one word per lane) and
 // clears them; then, for every word that had marks, it zeroes the word's slots as
 // consecutive 16-byte stores (512 B per warp store), lanes of unmarked units skipping
-// theirs, so the stores stay coalesced however the marks are spread.
+// theirs, so the stores stay coalesced however the marks are spread. Without marks every
+// unit is zeroed.
 __device__ __forceinline__ void clear_marked_warp(uint4* __restrict__ grad, int64_t total16,
                                                   int unit_shift, uint32_t* __restrict__ marks,
                                                   int64_t words, int64_t warp, int64_t warps,
@@ -260,8 +261,11 @@ __device__ __forceinline__ void clear_marked_warp(uint4* __restrict__ grad, int6
   const int slots = 32 << unit_shift;  // 16-byte slots under one word
   for (int64_t base = warp * 32; base < words; base += warps * 32) {
     const int64_t w = base + lane;
-    const uint32_t mine = w < words ? marks[w] : 0u;
-    if (mine != 0u) marks[w] = 0u;
+    uint32_t mine = w < words ? 0xffffffffu : 0u;
+    if (marks != nullptr) {
+      if (mine != 0u) mine = marks[w];
+      if (mine != 0u) marks[w] = 0u;
+    }
     uint32_t pending = __ballot_sync(kFull, mine != 0u);
     while (pending != 0u) {
       const int src = __ffs(pending) - 1;

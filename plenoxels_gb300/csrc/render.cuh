@@ -143,6 +143,12 @@ struct RenderArgs {
   const Real* target;
   Real* grad;
   uint32_t* grad_marks;  // optional: units of written gradient cells are marked here
+  // optional (fp32 training): another gradient buffer whose marked units are zeroed (without
+  // marks: the whole of it)
+  uint4* clear_grad;
+  int64_t clear_total16;
+  uint32_t* clear_marks;
+  int64_t clear_words;
   Real* loss_out;
   double* partials;  // fp64: block loss partials, and the block counter
   unsigned* counter;
@@ -1008,10 +1014,12 @@ render_kernel(const RenderArgs<Real> a) {
   __shared__ unsigned long long s_bins[2][kWarp];  // SUMS: the block's sums
   __shared__ unsigned s_special[2];
   __shared__ unsigned s_taken;  // QUEUE: rays of this block that have a warp
+  __shared__ unsigned s_cleared;  // SUMS: rounds of the clear that have a warp
   if (QUEUE || PHASE == kTrain) {
     if (threadIdx.x == 0) {
       s_done = 0u;
       s_taken = (unsigned)warps_per_block;
+      s_cleared = 0u;
     }
     if (SUMS && threadIdx.x < 2 * kWarp) s_bins[threadIdx.x >> 5][lane] = 0ull;
     if (SUMS && threadIdx.x < 2) s_special[threadIdx.x] = 0u;
@@ -1225,6 +1233,23 @@ render_kernel(const RenderArgs<Real> a) {
   }
 
   if constexpr (SUMS) {
+    // The other buffer's units are cleared by the warps that have run out of rays, 32 mark words
+    // at a time from a second counter of the block, while the block's last rays run. On a stream
+    // of its own the clear took the SMs that the kernel's blocks were waiting for, and two event
+    // waits a step: nearest steps of 3500 rays x 140..320 46 -> 27 and 50 -> 40 us, 512^3 log-sum
+    // 378 -> 338 us. Of the 8192-ray trilinear step's 101 us (256^3) the clear's 50 MB of zeros
+    // still are 15 and the marks 10; clearing along with each ray instead took 104 us.
+    if (a.clear_words > 0) {
+      const int64_t rounds = (a.clear_words + kWarp - 1) / kWarp;
+      for (;;) {
+        unsigned taken = 0;
+        if (lane == 0) taken = atomicAdd(&s_cleared, 1u);
+        const int64_t round = (int64_t)blockIdx.x + (int64_t)gridDim.x * __shfl_sync(kFull, taken, 0);
+        if (round >= rounds) break;
+        clear_marked_warp(a.clear_grad, a.clear_total16, kMarkCellsLog2, a.clear_marks, a.clear_words, round,
+                          rounds, lane);
+      }
+    }
     // Warps add their bins up in shared memory and the block's last warp adds them to the
     // launch's, so that a block fences once, at its end (a fence at device scope also empties
     // the SM's L1: one per warp took the nearest step of 8192 rays from 44 to 66 us). The last

@@ -36,8 +36,9 @@ int launch_render_k(const RenderArgs<Real>& a, cudaStream_t s) {
     resident = sms * per_sm;
     if (dev >= 0 && dev < 64) configured[dev] = resident;
   }
-  // fp32: one wave, or a ray per block when there are fewer rays; fp64: a ray per warp
-  int64_t blocks = a.R;
+  // fp32: one wave, or a ray per block when there are fewer rays (and nothing to clear beside
+  // them); fp64: a ray per warp
+  int64_t blocks = std::max<int64_t>(a.R, a.clear_words / kWarp);
   if (sizeof(Real) == 4)
     blocks = std::min<int64_t>(blocks, resident);
   else

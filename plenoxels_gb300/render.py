@@ -211,6 +211,12 @@ def camera_sample_indices(grid, transforms, images, camera_angle_x, num_rays, ra
     return idx, inb, coords
 
 
+# Smallest grid whose gradient units are marked (zeroing="marked"). Up to here zeroing the whole
+# buffer (32 MB) takes less than the marks' atomics on a bitmap of at most 64 KiB, where all
+# rays meet: %SMALL%.
+MARKED_CELLS = 1 << 21
+
+
 class FusedTrainStep:
     """Forward, MSE loss and backward of a batch of rays in one kernel launch.
 
@@ -225,14 +231,14 @@ class FusedTrainStep:
     unless zero_grad=False, in which case it accumulates like autograd does. Every call
     is asynchronous; the returned loss is a device scalar.
 
-    overlap_zero=True keeps two gradient buffers and zeroes the next step's buffer on a
-    side stream while the current step's kernel runs (the 256 MiB fill of a 256^3 grid
-    no longer sits on the critical path). A step's gradient then stays valid until the
+    overlap_zero=True keeps two gradient buffers and zeroes the next step's buffer while the
+    current step's kernel runs (the 256 MiB fill of a 256^3 grid no longer sits on the
+    critical path): on a side stream, or with zeroing="marked" in the kernel itself. A step's gradient then stays valid until the
     next step is launched; the buffer alternates, and ``grid.grad``/``self.grad`` follow.
 
     zeroing="marked" re-zeroes a gradient buffer by clearing only the 4-cell units its
     last step wrote (the kernel marks them in a bitmap of the buffer, pgb_clear_marked)
-    instead of writing the whole buffer. Every step still starts from an all-zero dense
+    instead of writing the whole buffer (grids of up to MARKED_CELLS cells are cleared whole). Every step still starts from an all-zero dense
     gradient, provided the caller only reads the gradient buffers (an optimizer that
     reads grid.grad, or zeroes it) and does not add into them; an in-place all-reduce of
     the gradient over ranks adds into them.
@@ -270,13 +276,15 @@ class FusedTrainStep:
         self._side = None
         if overlap_zero:
             self._grads.append(torch.zeros(grid.shape, dtype=self.real, device=dev))
-            self._side = torch.cuda.Stream(device=dev)
-            self._zeroed = [None, None]  # event: buffer b is zero and free
+            if zeroing != "marked":
+                self._side = torch.cuda.Stream(device=dev)
+            self._zeroed = [None, None]  # buffer b is zero and free: an event (fill), True (marked)
         if zeroing not in ("fill", "marked"):
             raise ValueError(f"zeroing must be 'fill' or 'marked', got {zeroing!r}")
         cells = grid.numel() // 4
+        self._marked = zeroing == "marked"
         self._marks = ([torch.zeros(lib.pgb_mark_words(cells), dtype=torch.int32, device=dev)
-                        for _ in self._grads] if zeroing == "marked" else None)
+                        for _ in self._grads] if self._marked and cells > MARKED_CELLS else None)
         self._cur = 0
         self._buf = 0  # index of the buffer the last launch wrote
         self.grad = self._grads[0]
@@ -303,9 +311,18 @@ class FusedTrainStep:
     def _gradient_for_step(self, zero_grad):
         if not zero_grad:
             return self.grad
-        if self._side is None:
+        if len(self._grads) == 1:
             self._fill(0, stream_of(self.grid))
             self._buf = 0
+            return self.grad
+        if self._side is None:
+            b = self._cur
+            if not self._zeroed[b]:
+                self._fill(b, stream_of(self.grid))
+            self._buf, self._cur = b, 1 - b
+            self._zeroed = [False, False]
+            self.grad = self._grads[b]
+            self._attach()
             return self.grad
         main = torch.cuda.current_stream(self.grid.device)
         b = self._cur
@@ -358,7 +375,15 @@ class FusedTrainStep:
             main = torch.cuda.current_stream(self.grid.device)
             ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
             ev[0].record(main)
-        if self.beta == 0.0:
+        if zero_grad and self._side is None and len(self._grads) == 2:
+            o = 1 - self._buf
+            terms = _lib.PgbLossTerms(self.loss_weight, self.beta, self.beta_eps)
+            check(lib.pgb_render_train_clear(gdesc, rdesc, ptr(target), terms, ptr(rgba_out), ptr(grad),
+                                             ptr(losses), ptr(self.workspace), ptr(self._grads[o]),
+                                             None if self._marks is None else ptr(self._marks[o]), stream),
+                  "train step")
+            self._zeroed[o] = True
+        elif self.beta == 0.0:
             check(lib.pgb_render_train(gdesc, rdesc, ptr(target), self.loss_weight, ptr(rgba_out),
                                        ptr(grad), ptr(losses), ptr(self.workspace), stream),
                   "train step")
