@@ -213,7 +213,8 @@ def camera_sample_indices(grid, transforms, images, camera_angle_x, num_rays, ra
 
 # Smallest grid whose gradient units are marked (zeroing="marked"). Up to here zeroing the whole
 # buffer (32 MB) takes less than the marks' atomics on a bitmap of at most 64 KiB, where all
-# rays meet: %SMALL%.
+# rays meet: steps of 48x79x72, 18,104 rays x 512 nearest 134 -> 52 us; 56x55x48, 16,045 x 141
+# nearest 124 -> 44 us; 105x113x124, 6430 x 267 trilinear 76 -> 44 us.
 MARKED_CELLS = 1 << 21
 
 
