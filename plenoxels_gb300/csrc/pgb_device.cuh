@@ -142,10 +142,12 @@ __device__ __forceinline__ Real warp_incl_prod(Real x, int lane) {
 
 // Inclusive suffix scan of affine maps f_l(s) = a_l + b_l * s composed towards lane 31:
 // after the call lane l holds F_l = f_l o f_{l+1} o ... o f_31 as (a, b).
+// from: the first step's distance.
 template <typename Real>
-__device__ __forceinline__ void warp_suffix_affine(Real& a, Real& b, int lane) {
+__device__ __forceinline__ void warp_suffix_affine(Real& a, Real& b, int lane, int from = 1) {
 #pragma unroll
   for (int d = 1; d < kWarp; d <<= 1) {
+    if (d < from) continue;
     const Real a2 = __shfl_down_sync(kFull, a, d);
     const Real b2 = __shfl_down_sync(kFull, b, d);
     if (lane + d < kWarp) {

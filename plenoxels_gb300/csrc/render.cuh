@@ -135,6 +135,7 @@ struct RenderArgs {
   int64_t first_ray;  // index of ray 0 in the stratification stream
   float term_thr;
   int chunk_samples;  // host-side chunk request (pick_slots)
+  int long_ray;    // the ray would be one long chunk (rounding of the suffix scan)
   int use_bg;      // rgb += (1 - A) * bg after compositing
   float bg[3];
   // outputs / adjoint inputs
@@ -542,11 +543,19 @@ __device__ __forceinline__ void sample_value(const GridP<Real>& g, Real nx, Real
   } else {
     // blend x, then y, then z, as src/grid_functions.py:34-42
     if constexpr (sizeof(Real) == 4) {
-      // channels in pairs, every operation rounded as below
+      // Products of channel pairs, every operation rounded as below. The sums are scalar ones:
+      // the assembler fuses a paired multiplication into a paired addition whatever their
+      // rounding suffixes say, and a blend an ulp away turns up as 6e-4 of a gradient where
+      // the beta term's 1 / (1 - alpha + eps) meets an opacity near 1. (Same time.)
       const F2 one = F2::of(1.f, 1.f);
       const F2 wx2 = F2::of(wx, wx), wy2 = F2::of(wy, wy), wz2 = F2::of(wz, wz);
       const F2 ux2 = sub2(one, wx2), uy2 = sub2(one, wy2), uz2 = sub2(one, wz2);
-      const auto blend = [](F2 a, F2 w, F2 b, F2 u) { return add2(mul2(a, w), mul2(b, u)); };
+      const auto blend = [](F2 a, F2 w, F2 b, F2 u) {
+        float p, q, r, s;
+        mul2(a, w).get(p, q);
+        mul2(b, u).get(r, s);
+        return F2::of(radd(p, r), radd(q, s));
+      };
 #pragma unroll
       for (int p = 0; p < 4; p += 2) {
         F2 a4[4];
@@ -1025,15 +1034,17 @@ render_kernel(const RenderArgs<Real> a) {
     if (SUMS && threadIdx.x < 2) s_special[threadIdx.x] = 0u;
     __syncthreads();
   }
+  const auto ray_of = [&](unsigned t) -> int64_t {  // the block's t-th ray
+    return (int64_t)blockIdx.x + (int64_t)gridDim.x * t;
+  };
   const auto next_ray = [&](int64_t r) -> int64_t {
     if (!QUEUE) return r + nw;
     unsigned taken = 0;
     if (lane == 0) taken = atomicAdd(&s_taken, 1u);
-    return (int64_t)blockIdx.x + (int64_t)gridDim.x * __shfl_sync(kFull, taken, 0);
+    return ray_of(__shfl_sync(kFull, taken, 0));
   };
 
-  for (int64_t r = QUEUE ? (int64_t)blockIdx.x + (int64_t)gridDim.x * (threadIdx.x >> 5) : gw; r < a.R;
-       r = next_ray(r)) {
+  for (int64_t r = QUEUE ? ray_of(threadIdx.x >> 5) : gw; r < a.R; r = next_ray(r)) {
     Ray<Real> ray;
     load_ray(a, r, ray, PHASE == kTrain);
     int first, end;
@@ -1201,7 +1212,21 @@ render_kernel(const RenderArgs<Real> a) {
         const Real al = vk[3];
         const Real G = gpx[0] * vk[0] + gpx[1] * vk[1] + gpx[2] * vk[2] + gpx[3];
         Real fa = G * al, fb = Real(1) - al;
-        warp_suffix_affine(fa, fb, lane);
+        if constexpr (MODE == PGB_NEAREST && K == 2 && sizeof(Real) == 4) {
+          // The first step's a + b * a2 with a = G * al has two fused forms, an ulp apart. Rays
+          // of 128 samples and more without early stop were one long chunk, whose code fuses
+          // the other product; their bits stay as they were (the beta term's 1 / (1 - alpha +
+          // eps) turns an ulp of an opacity near 1 into 6e-4 of the next step's gradient).
+          const Real a2 = __shfl_down_sync(kFull, fa, 1), b2 = __shfl_down_sync(kFull, fb, 1);
+          const Real near = rfma(fb, a2, fa), far = rfma(G, al, rmul(fb, a2));
+          if (lane < kWarp - 1) {
+            fa = a.long_ray ? far : near;
+            fb = fb * b2;
+          }
+          warp_suffix_affine(fa, fb, lane, 2);
+        } else {
+          warp_suffix_affine(fa, fb, lane);
+        }
         const Real S_here = fa + fb * Snext_carry;          // S_s for this lane's sample
         Real S_after = __shfl_down_sync(kFull, S_here, 1);  // S_{s+1}
         if (lane == kWarp - 1) S_after = Snext_carry;

@@ -59,13 +59,15 @@ int launch_render_mp(const RenderArgs<Real>& a, cudaStream_t s) {
     if (!a.g.quick) return launch_render_k<Real, Store, MODE, 8, PHASE, LOGT, kGeneral>(a, s);
   }
   const bool early_stop = a.g.clip && !(PHASE == kTrain && a.beta_w != 0.0);
+  RenderArgs<Real> b = a;
+  b.long_ray = MODE == PGB_NEAREST && !early_stop && a.chunk_samples <= 0 && a.S > 128;
   const bool long_chunks = long_chunks_for(a.S, MODE, early_stop, PHASE != kForward, a.term_thr);
   switch (pick_slots(a.S, a.chunk_samples, MODE, long_chunks)) {
-    case 1: return launch_render_k<Real, Store, MODE, 1, PHASE, LOGT, A>(a, s);
-    case 2: return launch_render_k<Real, Store, MODE, 2, PHASE, LOGT, A>(a, s);
-    case 4: return launch_render_k<Real, Store, MODE, 4, PHASE, LOGT, A>(a, s);
-    case 8: return launch_render_k<Real, Store, MODE, 8, PHASE, LOGT, A>(a, s);
-    case 16: return launch_render_k<Real, Store, MODE, 16, PHASE, LOGT, A>(a, s);
+    case 1: return launch_render_k<Real, Store, MODE, 1, PHASE, LOGT, A>(b, s);
+    case 2: return launch_render_k<Real, Store, MODE, 2, PHASE, LOGT, A>(b, s);
+    case 4: return launch_render_k<Real, Store, MODE, 4, PHASE, LOGT, A>(b, s);
+    case 8: return launch_render_k<Real, Store, MODE, 8, PHASE, LOGT, A>(b, s);
+    case 16: return launch_render_k<Real, Store, MODE, 16, PHASE, LOGT, A>(b, s);
     default: return PGB_ERR_UNSUPPORTED;
   }
 }
