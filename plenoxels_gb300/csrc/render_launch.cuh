@@ -45,7 +45,14 @@ int launch_render_k(const RenderArgs<Real>& a, cudaStream_t s) {
     blocks = std::min<int64_t>((a.R + kWarpsPerBlock - 1) / kWarpsPerBlock,
                                PHASE == kTrain ? kMaxTrainWarps / kWarpsPerBlock : (int64_t)1 << 20);
   if (blocks < 1) blocks = 1;
-  render_kernel<Real, Store, MODE, K, PHASE, LOGT, A><<<(unsigned)blocks, kThreads, kSmem, s>>>(a);
+  // Groups of up to 8 consecutive rays as long as every block gets at least 32 groups (one more
+  // or less is little then; training batches of some thousand rays keep single rays):
+  // neighbouring rays of a picture share cells. One 800 x 800 picture of a 256^3 grid in
+  // groups of 1 / 8 / 32 / 128: 976 / 792 / 776 / 797 us, three of 400 x 400: 678 / 648 / 677
+  // / 676 us, half transparent 1913 / 1625 / 1630 / 1635 us.
+  RenderArgs<Real> b = a;
+  while (b.group_log2 < 3 && (a.R >> (b.group_log2 + 1)) >= 32 * blocks) ++b.group_log2;
+  render_kernel<Real, Store, MODE, K, PHASE, LOGT, A><<<(unsigned)blocks, kThreads, kSmem, s>>>(b);
   return after_launch();
 }
 
