@@ -6,7 +6,7 @@ from a second seeded ground-truth grid; 8192 random rays per step spread camera-
 the cameras, near 2, far 6, 256 stratified samples per ray, trilinear lookup). Synthetic
 seeded data stands in for the NeRF-synthetic scenes.
 
-A step = zero the dense gradient (on a side stream, by clearing the cells the buffer's
+A step = zero the dense gradient (the kernel clears the other buffer, the cells its
 previous step wrote) + one fused kernel that generates the rays from the resident cameras
 and images, samples, looks up, composites, takes the MSE gradient and scatters dL/dcell. `value` is rays/s with everything resident in HBM; `e2e` is the same
 metric through FusedTrainStep.step_rays with the ray batch (origins, dirs, targets)
@@ -467,8 +467,9 @@ def full_step_leg(pg, grid, T, imgs, W, dev, steps, warmup):
     t1.record(stream)
     torch.cuda.synchronize(dev)
     ms = t0.elapsed_time(t1) / steps
-    # the Adam pass alone: reads param, grad, both moments and the accumulator, writes all
-    # five back (the gradient as zeros): 10 x 16 B per cell
+    # the Adam pass alone, on a gradient of zeros after the first: cells whose moments are not 0
+    # are read and written (param, both moments) and their gradient is read, 7 x 16 B; the
+    # 10 x 16 B of a cell that has a gradient are the yardstick
     a0, a1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     a0.record(stream)
     for _ in range(steps):
@@ -479,6 +480,9 @@ def full_step_leg(pg, grid, T, imgs, W, dev, steps, warmup):
     adam_bytes = grid.numel() // 4 * 160
     # the TV loss reduction + the Adam pass with the TV stencil fused (what a step runs)
     bufs = [tr.grid, tr._spare if tr._spare is not None else torch.empty_like(tr.grid)]
+    tr.opt.step_tv(tr.render.grad, 1e-5, bufs[1])  # warm-up (torch loads the sqrt of its value)
+    bufs.reverse()
+    torch.cuda.synchronize(dev)
     a0.record(stream)
     for i in range(steps):
         tr.opt.step_tv(tr.render.grad, 1e-5, bufs[(i + 1) % 2])

@@ -53,8 +53,12 @@ int launch_render_logt_bf16(const RenderArgs<float>& a, int mode, int phase, cud
 // beta term, no clip). Measured on GB300, one training launch, chunks of 32 / 64 / 128 / 256
 // samples: 256^3 trilinear, 8192 rays x 256 with early stop 80 / 96 / 105 / 162 us; 7500
 // rays x 600 with the beta term trilinear 359 / 380 / 403 / 569 us, nearest 146 / 132 / 134
-// / 189 us (256 was the choice there before); nearest without it 105 / 92 / 92 / 127 us.
-// `long_chunks` (long_chunks_for) keeps whole rays up to 512 samples in one chunk.
+// / 189 us (256 was the choice there before); nearest without it 105 / 92 / 92 / 127 us. With
+// the queue of rays, 8192 rays x 256 with the beta term, opaque, trilinear: 137 / 138 / 237 /
+// 277 us (172 before it in one chunk); 200^3 without clip, 64 / 128 / 256 samples: 80 / 126 /
+// 169 us in chunks of 32 and 80 / 131 / 206 us in one.
+// `long_chunks` keeps whole rays up to 512 samples in one chunk: rays that may not stop early
+// and have a threshold on T, which is looked at after each chunk.
 inline int pick_slots(int S, int chunk_samples = 0, int mode = PGB_TRILINEAR,
                       bool long_chunks = false) {
 #ifdef PGB_FORCE_SLOTS
@@ -66,15 +70,6 @@ inline int pick_slots(int S, int chunk_samples = 0, int mode = PGB_TRILINEAR,
   while (k < 16 && 32 * k < chunk_samples) k *= 2;
   while (k < 16 && (S + 32 * k - 1) / (32 * k) > kMaxChunks) k *= 2;
   return k;
-}
-
-// Long chunks where a ray may not stop early, (a) with a threshold on T, which is looked at
-// after each chunk, and (b) for the trilinear gradient of up to 256 samples, where there is
-// nothing to skip and one gather of the ray keeps the most loads in flight (8192 rays of 64 /
-// 128 / 256 samples, 200^3, no clip: 78 / 126 / 185 us against 85 / 139 / 190 us in chunks
-// of 32).
-inline bool long_chunks_for(int S, int mode, bool early_stop, bool gradient, float term_threshold) {
-  return !early_stop && (term_threshold > 0.f || (mode == PGB_TRILINEAR && gradient && S <= 256));
 }
 
 }  // namespace pgb

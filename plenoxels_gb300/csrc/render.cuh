@@ -724,8 +724,9 @@ __device__ __forceinline__ void warp_merged_scatter(const GridP<Real>& g, Real* 
 // two of 16 warps took 76 us for 71 at 7500 rays x 600, 85 before the queue); trilinear
 // lookup with 32-sample chunks two blocks of 12 warps for the gradient (80 registers; one of
 // 24 warps the same within 2 %, six of 4 warps 345 us for 333) and two of 14 for a forward
-// pass (72 registers). Longer trilinear chunks need 90 to 210 registers: 8 warps a block, as
-// many blocks as fit. fp64 launches have a ray per warp, in blocks of 4 or 8 warps.
+// pass (72 registers). Longer trilinear chunks need 90 to 210 registers: 8 warps a block, two
+// blocks of up to 256-sample chunks per SM (8192 rays x 256 with the beta term: 277 us with
+// one, 185 with two). fp64 launches have a ray per warp, in blocks of 4 or 8 warps.
 #ifndef PGB_RENDER_THREADS
 #define PGB_RENDER_THREADS 256
 #endif
@@ -976,7 +977,7 @@ template <typename Real, int MODE, int K, int PHASE>
 constexpr int render_min_blocks() {
   if (sizeof(Real) != 4) return MODE == PGB_NEAREST ? 4 : (K == 1 ? 6 : 0);
   return MODE == PGB_NEAREST ? 1024 / PGB_RENDER_THREADS_NEAREST
-         : K != 1 ? 0
+         : K != 1 ? (K <= 8 ? 2 : 0)
          : PHASE == kForward ? 896 / PGB_RENDER_THREADS_FWD : 768 / PGB_RENDER_THREADS_K1;
 }
 
