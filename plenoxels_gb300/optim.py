@@ -47,6 +47,8 @@ class FusedAdam:
         returns the term's value as a device scalar. grid defaults to the optimised grid
         (the pooled grid while progressive growing runs)."""
         self._tv_pass(grad, weight, self.grid if grid is None else grid)
+        if not grad.is_inference():
+            torch.autograd.graph.increment_version(grad)
         return float(weight) * self.tv_sumsq.sqrt()
 
     @torch.no_grad()

@@ -294,6 +294,7 @@ class FusedTrainStep:
         self.loss = self.losses[0]
         self._attach()
         self._cams = None
+        self.launches = 0  # steps launched; each writes to the gradient
         self.kernel_events = None  # list of (start, end) CUDA events, when timing is wanted
 
     def _attach(self):
@@ -366,6 +367,7 @@ class FusedTrainStep:
     def _launch(self, rdesc, target, rgba_out, zero_grad, loss_out=None):
         lib = _lib.load()
         losses = self._loss_target(loss_out)
+        self.launches += 1
         grad = self._gradient_for_step(zero_grad)
         if self._marks is not None:
             rdesc.grad_marks = ptr(self._marks[self._buf])

@@ -13,8 +13,10 @@ place, at the cost of the separate TV gradient pass).
 Progressive growing (scripts/train.py:91-123): while the schedule's receptive field r is
 above 1, the step renders the grid average-pooled with window r and stride max(1, r//4)
 (pitch points_distance * stride, origin at the coordinate of cell r//2), and the pooled
-gradient is spread back onto the full grid by the pooling's adjoint inside the Adam pass
-(the full gradient stays zero). The TV term applies once r < 19, to the grid being rendered.
+gradient is spread back onto the full grid by the pooling's adjoint inside the Adam pass.
+The full gradient is zero after every step: a pooled step leaves it alone unless it was
+written since the last step, and the last pooled step zeroes it whatever was seen of it.
+The TV term applies once r < 19, to the grid being rendered.
 """
 from __future__ import annotations
 
@@ -54,8 +56,9 @@ class Trainer:
         self.step_index = 0
         self._pooled = {}  # field -> (pooled grid, its FusedTrainStep, stride, scratch)
         self.losses = torch.zeros(3, device=grid.device)  # mse, tv, beta of the last step
-        # the full gradient is all zeros between steps, unless the caller writes to it
-        self._grad_version = self.render.grad._version
+        # the full gradient is all zeros after a step; the state tells whether it was written since
+        self._grad_state = self._full_grad_state()
+        self._unseen = False  # pooled steps ran since it was last zeroed: a write may have gone unseen
 
     def field(self, i):
         """Receptive field of step i (scripts/train.py:108); 0 once the schedule ends."""
@@ -76,6 +79,18 @@ class Trainer:
             self._pooled[r] = (pooled, step, stride, scratch)
         return self._pooled[r]
 
+    def _full_grad_state(self):
+        """Changes with every launch of self.render and every write that torch counts (torch's
+        operators, FusedAdam.add_tv). Writes through raw pointers or .data change nothing. None
+        where torch counts none (a trainer made in inference mode)."""
+        g = self.render.grad
+        return None if g.is_inference() else (self.render.launches, g._version)
+
+    def _zero_full_grad(self, s):
+        g = self.render.grad
+        check(_lib.load().pgb_fill_zero(ptr(g), g.numel() * g.element_size(), s), "train step")
+        self._unseen = False
+
     def _run(self, launch):
         r = self.field(self.step_index) if self.progressive else 0
         lib = _lib.load()
@@ -90,6 +105,8 @@ class Trainer:
             render_step, tv_grid, tv_grad = step, pooled, step.grad
         else:
             # the Adam pass left the gradient zeroed: accumulate into it directly
+            if self._unseen:
+                self._zero_full_grad(s)
             launch(self.render, False)
             render_step, tv_grid, tv_grad = self.render, self.grid, full_grad
         if self.tv > 0.0 and r < 19 and self.fuse_tv and r <= 1:
@@ -105,13 +122,16 @@ class Trainer:
         with_tv = self.tv > 0.0 and r < 19
         if with_tv:
             self.opt._tv_pass(tv_grad, self.tv, tv_grid)
-        if r > 1 and full_grad._version == self._grad_version:
+        state = self._full_grad_state()
+        if r > 1 and state is not None and state == self._grad_state:
             self.opt.step_pooled(render_step.grad, r, stride, scratch)
+            self._unseen = True
+            if self.field(self.step_index + 1) <= 1:
+                self._zero_full_grad(s)
         else:
-            if r > 1:  # the caller wrote to the full gradient: the step overwrites and zeroes it
+            if r > 1:  # the full gradient was written: the step overwrites and zeroes it
                 check(lib.pgb_avg_pool3d_bwd(ptr(render_step.grad), _lib.dims3(self.grid.shape), r,
                                              stride, ptr(scratch), ptr(full_grad), s), "pooled grid")
-                self._grad_version = full_grad._version
             self.opt.step(full_grad)
         return self._finish(render_step, with_tv, s)
 
@@ -121,6 +141,7 @@ class Trainer:
         check(_lib.load().pgb_step_losses(ptr(render_step.losses), ptr(self.opt.tv_sumsq) if with_tv else None,
                                           self.tv, 1 if self.beta != 0.0 else 0, ptr(self.losses), s),
               "train step")
+        self._grad_state = self._full_grad_state()
         self.step_index += 1
         return self.losses
 
