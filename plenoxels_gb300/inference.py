@@ -20,7 +20,7 @@ from . import _lib
 from ._lib import check, ptr, require_cuda, stream_of
 from .grid_functions import grid_origin
 from .ray_sampling import _f32, generate_rays_batched
-from .render import _check_rays, _rays_desc, _render_cfg, _render_forward
+from .render import _check_rays, _rays_desc, _render, _render_cfg
 
 PARAM_KEYS = ("device", "number_of_rays", "num_samples", "delta_step", "even_spread",
               "camera_ray", "points_distance", "gridsize")
@@ -114,5 +114,5 @@ def render_camera_images(grid, transforms, height, width, camera_angle_x, near, 
                                     ptr(pixels), None, stream_of(T)), "render_camera_images")
         origins = (T[0, :3, 3] + near * dirs).contiguous()
         _check_rays(g, origins, dirs)
-        _render_forward(g, origins, dirs, cfg, out[c])
+        _render(g, origins, dirs, cfg, out[c].view(R, 4))
     return out

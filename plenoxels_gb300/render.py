@@ -90,8 +90,12 @@ def _render_forward(grid, origins, dirs, cfg, rgba=None):
 
 def _wants_autograd(*tensors):
     """Whether a call has to go through its autograd Function: a gradient may be asked for,
-    or a transform (vmap, forward-mode, functional tracing) is at work and decides itself."""
+    a transform (vmap, forward-mode, functional tracing) is at work and decides itself, or the
+    call is being traced (a trace records the Function as one operator, and a launch through a
+    pointer not at all)."""
     if torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0:
+        return True
+    if torch.jit.is_tracing():
         return True
     return torch.is_grad_enabled() and any(t.requires_grad for t in tensors)
 
@@ -139,10 +143,15 @@ def render_rays(grid, origins, dirs, delta_step, num_samples, points_distance, g
         grid_min = grid_origin(grid.shape, points_distance, _lib.real_dtype(grid.dtype))
     cfg = _render_cfg(grid_min, points_distance, mode, delta_step, num_samples, clip, stratified, seed,
                       term_threshold, background, transmittance, chunk_samples)
-    grid, origins, dirs = grid.contiguous(), origins.contiguous(), dirs.contiguous()
+    return _render(grid.contiguous(), origins.contiguous(), dirs.contiguous(), cfg)
+
+
+def _render(grid, origins, dirs, cfg, rgba=None):
+    """The checked rays' pixels; rgba: a contiguous [R,4] tensor for them (no gradient then)."""
     if not _wants_autograd(grid, origins, dirs):
-        return _render_forward(grid, origins, dirs, cfg)
-    return _RenderRays.apply(grid, origins, dirs, cfg)
+        return _render_forward(grid, origins, dirs, cfg, rgba)
+    out = _RenderRays.apply(grid, origins, dirs, cfg)
+    return out if rgba is None else rgba.copy_(out)
 
 
 def render_sample_indices(grid, origins, dirs, delta_step, num_samples, points_distance,
