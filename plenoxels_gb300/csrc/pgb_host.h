@@ -45,6 +45,11 @@ int launch_render_f64(const RenderArgs<double>& a, int mode, int phase, cudaStre
 // Log-sum transmittance form (fp32 arithmetic over fp32 or BF16 cells).
 int launch_render_logt_f32(const RenderArgs<float>& a, int mode, int phase, cudaStream_t s);
 int launch_render_logt_bf16(const RenderArgs<float>& a, int mode, int phase, cudaStream_t s);
+// fp32 and BF16 grids outside the quick index arithmetic's range (quick_grid).
+int launch_render_general_f32(const RenderArgs<float>& a, int mode, int phase, cudaStream_t s);
+int launch_render_general_bf16(const RenderArgs<float>& a, int mode, int phase, cudaStream_t s);
+int launch_render_general_logt_f32(const RenderArgs<float>& a, int mode, int phase, cudaStream_t s);
+int launch_render_general_logt_bf16(const RenderArgs<float>& a, int mode, int phase, cudaStream_t s);
 
 // Slots per lane (K) of a chunk of 32 * K samples. A chunk size (32 * K for K in 1, 2, 4, 8,
 // 16) is raised until a ray spans at most kMaxChunks chunks. Without a requested one: 32

@@ -113,11 +113,13 @@ template <>
 inline int dispatch_render<float>(const pgb_grid* g, const pgb_rays* r, RenderArgs<float>& a, int phase,
                            cudaStream_t s) {
   finish_args(a);
-  if (r->log_transmittance)
-    return g->dtype == PGB_BF16 ? launch_render_logt_bf16(a, g->mode, phase, s)
-                                : launch_render_logt_f32(a, g->mode, phase, s);
-  return g->dtype == PGB_BF16 ? launch_render_bf16(a, g->mode, phase, s)
-                              : launch_render_f32(a, g->mode, phase, s);
+  using Launch = int (*)(const RenderArgs<float>&, int, int, cudaStream_t);
+  static constexpr Launch kLaunch[2][2][2] = {  // [quick][log-sum][BF16]
+      {{launch_render_general_f32, launch_render_general_bf16},
+       {launch_render_general_logt_f32, launch_render_general_logt_bf16}},
+      {{launch_render_f32, launch_render_bf16}, {launch_render_logt_f32, launch_render_logt_bf16}}};
+  return kLaunch[a.g.quick ? 1 : 0][r->log_transmittance ? 1 : 0][g->dtype == PGB_BF16 ? 1 : 0](
+      a, g->mode, phase, s);
 }
 template <>
 inline int dispatch_render<double>(const pgb_grid* g, const pgb_rays* r, RenderArgs<double>& a, int phase,

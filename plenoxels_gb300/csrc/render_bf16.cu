@@ -3,6 +3,6 @@
 
 namespace pgb {
 int launch_render_bf16(const RenderArgs<float>& a, int mode, int phase, cudaStream_t s) {
-  return launch_render_t<float, __nv_bfloat16>(a, mode, phase, s);
+  return launch_render_t<float, __nv_bfloat16, false, kQuick>(a, mode, phase, s);
 }
 }  // namespace pgb

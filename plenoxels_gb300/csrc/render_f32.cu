@@ -3,6 +3,6 @@
 
 namespace pgb {
 int launch_render_f32(const RenderArgs<float>& a, int mode, int phase, cudaStream_t s) {
-  return launch_render_t<float, float>(a, mode, phase, s);
+  return launch_render_t<float, float, false, kQuick>(a, mode, phase, s);
 }
 }  // namespace pgb

@@ -3,6 +3,6 @@
 
 namespace pgb {
 int launch_render_f64(const RenderArgs<double>& a, int mode, int phase, cudaStream_t s) {
-  return launch_render_t<double, double>(a, mode, phase, s);
+  return launch_render_t<double, double, false, kGeneral>(a, mode, phase, s);
 }
 }  // namespace pgb

@@ -1,0 +1,8 @@
+// BF16 grids outside the quick index arithmetic's range (quick_grid).
+#include "render_launch.cuh"
+
+namespace pgb {
+int launch_render_general_bf16(const RenderArgs<float>& a, int mode, int phase, cudaStream_t s) {
+  return launch_render_t<float, __nv_bfloat16, false, kGeneral>(a, mode, phase, s);
+}
+}  // namespace pgb

@@ -56,15 +56,8 @@ int launch_render_k(const RenderArgs<Real>& a, cudaStream_t s) {
   return after_launch();
 }
 
-template <typename Real, typename Store, int MODE, int PHASE, bool LOGT>
+template <typename Real, typename Store, int MODE, int PHASE, bool LOGT, int A>
 int launch_render_mp(const RenderArgs<Real>& a, cudaStream_t s) {
-  // Grids outside the quick index arithmetic's range (a dimension of one cell or above
-  // 2^21, 2^32 cells): one kernel with the general arithmetic serves every ray length.
-  // fp64 grids have the general arithmetic throughout.
-  constexpr int A = sizeof(Real) == 4 ? kQuick : kGeneral;
-  if constexpr (A == kQuick) {
-    if (!a.g.quick) return launch_render_k<Real, Store, MODE, 8, PHASE, LOGT, kGeneral>(a, s);
-  }
   const bool early_stop = a.g.clip && !(PHASE == kTrain && a.beta_w != 0.0);
   RenderArgs<Real> b = a;
   b.long_ray = MODE == PGB_NEAREST && !early_stop && a.chunk_samples <= 0 && a.S > 128;
@@ -79,16 +72,22 @@ int launch_render_mp(const RenderArgs<Real>& a, cudaStream_t s) {
   }
 }
 
-template <typename Real, typename Store, bool LOGT = false>
+// A: kQuick for the fp32 grids of quick_grid, kGeneral for all others and for fp64. Both have
+// every chunk size: chunk_samples and the threshold on T mean the same on any grid. Origin (0,
+// 0, 0) against the same grid centred, us, general / quick (one general kernel of 256-sample
+// chunks for all took the figure behind): 256^3, 8192 rays x 256 trilinear step 102 / 99 (198);
+// 512^3 BF16 log-sum step of 65,536 rays 279 / 277 (1897); nearest, 7500 x 600 62 / 57 (102);
+// 160,000 rays x 256 forward, trilinear 304 / 300 (1139), nearest 260 / 253 (332).
+template <typename Real, typename Store, bool LOGT, int A>
 int launch_render_t(const RenderArgs<Real>& a, int mode, int phase, cudaStream_t s) {
   if (mode == PGB_NEAREST) {
-    if (phase == kForward) return launch_render_mp<Real, Store, PGB_NEAREST, kForward, LOGT>(a, s);
-    if (phase == kBackward) return launch_render_mp<Real, Store, PGB_NEAREST, kBackward, LOGT>(a, s);
-    if (phase == kTrain) return launch_render_mp<Real, Store, PGB_NEAREST, kTrain, LOGT>(a, s);
+    if (phase == kForward) return launch_render_mp<Real, Store, PGB_NEAREST, kForward, LOGT, A>(a, s);
+    if (phase == kBackward) return launch_render_mp<Real, Store, PGB_NEAREST, kBackward, LOGT, A>(a, s);
+    if (phase == kTrain) return launch_render_mp<Real, Store, PGB_NEAREST, kTrain, LOGT, A>(a, s);
   } else if (mode == PGB_TRILINEAR) {
-    if (phase == kForward) return launch_render_mp<Real, Store, PGB_TRILINEAR, kForward, LOGT>(a, s);
-    if (phase == kBackward) return launch_render_mp<Real, Store, PGB_TRILINEAR, kBackward, LOGT>(a, s);
-    if (phase == kTrain) return launch_render_mp<Real, Store, PGB_TRILINEAR, kTrain, LOGT>(a, s);
+    if (phase == kForward) return launch_render_mp<Real, Store, PGB_TRILINEAR, kForward, LOGT, A>(a, s);
+    if (phase == kBackward) return launch_render_mp<Real, Store, PGB_TRILINEAR, kBackward, LOGT, A>(a, s);
+    if (phase == kTrain) return launch_render_mp<Real, Store, PGB_TRILINEAR, kTrain, LOGT, A>(a, s);
   }
   return PGB_ERR_ARG;
 }

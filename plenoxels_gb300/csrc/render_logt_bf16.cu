@@ -4,6 +4,6 @@
 
 namespace pgb {
 int launch_render_logt_bf16(const RenderArgs<float>& a, int mode, int phase, cudaStream_t s) {
-  return launch_render_t<float, __nv_bfloat16, true>(a, mode, phase, s);
+  return launch_render_t<float, __nv_bfloat16, true, kQuick>(a, mode, phase, s);
 }
 }  // namespace pgb

@@ -5,6 +5,6 @@
 
 namespace pgb {
 int launch_render_logt_f32(const RenderArgs<float>& a, int mode, int phase, cudaStream_t s) {
-  return launch_render_t<float, float, true>(a, mode, phase, s);
+  return launch_render_t<float, float, true, kQuick>(a, mode, phase, s);
 }
 }  // namespace pgb
