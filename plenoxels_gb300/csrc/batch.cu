@@ -72,12 +72,13 @@ struct BatchArgs {
   float* rgba_out;
   float* loss_out;
   unsigned long long* work;  // ray queue head
+  unsigned long long* work_others;  // of the second queue
   unsigned* ticket;          // finished blocks
   float* ray_loss;           // [R] squared error per ray
 };
 
-// Workspace: the queue head (8 B), the finished-block ticket (4 B) and the loss sum's
-// ticket (4 B) in the first 64 B, then the loss sum's block partials, then one float per
+// Workspace: the queue head (8 B), the finished-block ticket (4 B), the loss sum's ticket (4 B)
+// and the second queue's head (8 B) in the first 64 B, then the loss sum's block partials, then one float per
 // ray.
 constexpr int kLossBlocks = 1024;
 constexpr int64_t kLossPartialsOffset = 64;
@@ -155,17 +156,38 @@ using BatchStage = ChunkStage<float, K, (K == 1 ? PGB_BATCH_STAGE_CHUNKS : 1),
 // Bytes of one warp's scene arguments in shared memory (the stage behind them stays aligned).
 constexpr int kSceneArgsBytes = ((int)sizeof(RenderArgs<float>) + 15) & ~15;
 
+// A scene that leaves the quick arithmetic's range by an origin component near 0 alone (a
+// scene in [0, 1]^3, an axis of one or two cells) is scaled by 2^24, its rays with it: every
+// position, difference and quotient comes out as without, rounding included, as long as
+// neither underflows, and a normal difference is then as far from underflow as the two
+// corrections of div_pd need it. (Positions of 2^104 overflow, which no grid in range holds.)
+// Trilinear lookup only: for nearest lookup the general arithmetic costs less than a loop apart.
+constexpr float kSceneScale = 16777216.0f;
+enum SceneArith { kSceneGeneral = 0, kSceneQuick = 1, kSceneScaled = 2 };  // GridP::quick
+
+template <int MODE>
+__device__ __forceinline__ SceneArith scene_arith(const pgb_scene& sc) {
+  const auto off_zero = [](float o) { return fabsf(o) < kQuickMinOrigin ? kQuickMinOrigin : o; };
+  const float* o = sc.origin;
+  const int X = sc.dims[0], Y = sc.dims[1], Z = sc.dims[2];
+  if (quick_grid(X, Y, Z, o[0], o[1], o[2], sc.points_distance)) return kSceneQuick;
+  return MODE == PGB_TRILINEAR &&
+                 quick_grid(X, Y, Z, off_zero(o[0]), off_zero(o[1]), off_zero(o[2]), sc.points_distance)
+             ? kSceneScaled : kSceneGeneral;
+}
+
 // A scene as the single-scene kernels see it.
+template <int MODE>
 __device__ __forceinline__ void scene_args(const BatchArgs& a, const pgb_scene& sc,
                                            RenderArgs<float>& ra) {
   ra.g.cells = sc.cells;
   ra.g.X = sc.dims[0]; ra.g.Y = sc.dims[1]; ra.g.Z = sc.dims[2];
   ra.g.fX = (float)sc.dims[0]; ra.g.fY = (float)sc.dims[1]; ra.g.fZ = (float)sc.dims[2];
-  ra.g.ox = sc.origin[0]; ra.g.oy = sc.origin[1]; ra.g.oz = sc.origin[2];
-  ra.g.pd = sc.points_distance;
-  ra.g.inv_pd = 1.0f / sc.points_distance;
-  ra.g.quick = quick_grid(sc.dims[0], sc.dims[1], sc.dims[2], sc.origin[0], sc.origin[1],
-                          sc.origin[2], sc.points_distance) ? 1 : 0;
+  ra.g.quick = scene_arith<MODE>(sc);
+  const float scale = ra.g.quick == kSceneScaled ? kSceneScale : 1.0f;
+  ra.g.ox = scale * sc.origin[0]; ra.g.oy = scale * sc.origin[1]; ra.g.oz = scale * sc.origin[2];
+  ra.g.pd = scale * sc.points_distance;
+  ra.g.inv_pd = 1.0f / ra.g.pd;
   ra.g.clip = a.clip;
   ra.g.alpha_floor = 0.f;
   ra.S = sc.num_samples;
@@ -176,16 +198,21 @@ __device__ __forceinline__ void scene_args(const BatchArgs& a, const pgb_scene& 
 
 // One ray of the batch: sampling, lookup, compositing, squared error and adjoint on its own
 // scene. MERGE: the trilinear scatter merges the warp's updates of the same cell
-// (warp_merged_scatter) before its atomics. A: the index arithmetic (Arith).
-template <typename Store, int MODE, int K, bool MERGE, int A>
+// (warp_merged_scatter) before its atomics. ARITH: the scene's arithmetic (SceneArith).
+template <typename Store, int MODE, int K, bool MERGE, int ARITH>
 __device__ __forceinline__ void batch_ray(const BatchArgs& a, const pgb_scene& sc,
                                           const RenderArgs<float>& ra, int64_t r, BatchStage<K> cs,
                                           int lane) {
+  constexpr int A = ARITH == kSceneGeneral ? kGeneral : kQuick;
   const float grad_scale = a.grad_scale;  // d(weighted MSE)/d pixel
   float* grad = ra.grad;
   Ray<float> ray;
   ray.ox = a.origins[3 * r + 0]; ray.oy = a.origins[3 * r + 1]; ray.oz = a.origins[3 * r + 2];
   ray.dx = a.dirs[3 * r + 0];    ray.dy = a.dirs[3 * r + 1];    ray.dz = a.dirs[3 * r + 2];
+  if constexpr (ARITH == kSceneScaled) {
+    ray.ox *= kSceneScale; ray.oy *= kSceneScale; ray.oz *= kSceneScale;
+    ray.dx *= kSceneScale; ray.dy *= kSceneScale; ray.dz *= kSceneScale;
+  }
   ray.tgt = a.target[4 * r + (lane & 3)];
   ray.h = a.stratified ? hash_stream(a.seed, (uint64_t)r) : 0ull;
 
@@ -336,22 +363,42 @@ __device__ __forceinline__ void batch_ray(const BatchArgs& a, const pgb_scene& s
   }
 }
 
-// Scenes outside the quick index arithmetic's range go through a call of their own, so
-// that the kernel's registers are those of the quick form (with both forms inline, its 80
-// registers spilled 264 bytes).
+// The kernel's shared memory: the scene table, per warp the arguments of the scene that its ray
+// belongs to, and the stages.
+template <int K>
+struct BatchShared {
+  pgb_scene* scenes;
+  // rewritten when a ray of another scene comes; read where they are used: as local variables
+  // they and their spills took 140 bytes of stack in the 80-register kernel
+  RenderArgs<float>* args;
+  BatchStage<K> stage;
+  __device__ __forceinline__ BatchShared(unsigned char* smem, int num_scenes)
+      : scenes(reinterpret_cast<pgb_scene*>(smem)),
+        args(reinterpret_cast<RenderArgs<float>*>(smem + table_bytes(num_scenes) +
+                                                  (size_t)(threadIdx.x >> 5) * kSceneArgsBytes)),
+        stage(smem + table_bytes(num_scenes) + (size_t)kSceneArgsBytes * (blockDim.x / kWarp),
+              threadIdx.x >> 5) {}
+  __host__ __device__ static constexpr size_t table_bytes(int num_scenes) {
+    return ((size_t)num_scenes * sizeof(pgb_scene) + 15) & ~(size_t)15;
+  }
+};
+
+// A ray of a scene in the general arithmetic, by a call of its own that finds the shared memory
+// again by itself (through pointers it was not known to be shared: 1923 us for 1792, a step of
+// 16 such scenes).
 template <typename Store, int MODE, int K, bool MERGE>
-__device__ __noinline__ void batch_ray_general(const BatchArgs& a, const pgb_scene& sc,
-                                               const RenderArgs<float>& ra, int64_t r,
-                                               BatchStage<K> cs, int lane) {
-  batch_ray<Store, MODE, K, MERGE, kGeneral>(a, sc, ra, r, cs, lane);
+__device__ __noinline__ void batch_ray_general(const BatchArgs& a, int sid, int64_t r, int lane) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const BatchShared<K> sh(smem_raw, a.num_scenes);
+  batch_ray<Store, MODE, K, MERGE, kSceneGeneral>(a, sh.scenes[sid], *sh.args, r, sh.stage, lane);
 }
 
 template <typename Store, int MODE, int K, bool MERGE>
 __global__ void __launch_bounds__(kBatchMaxThreads, K == 1 ? PGB_BATCH_MIN_BLOCKS_K1 : PGB_BATCH_MIN_BLOCKS)
     batch_train_kernel(const __grid_constant__ BatchArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  pgb_scene* sc_tab = reinterpret_cast<pgb_scene*>(smem_raw);
-  const size_t tab_bytes = ((size_t)a.num_scenes * sizeof(pgb_scene) + 15) & ~(size_t)15;
+  const BatchShared<K> sh(smem_raw, a.num_scenes);
+  RenderArgs<float>& ra = *sh.args;
   {
     const uint32_t* src = reinterpret_cast<const uint32_t*>(a.scenes);
     uint32_t* dst = reinterpret_cast<uint32_t*>(smem_raw);
@@ -360,39 +407,51 @@ __global__ void __launch_bounds__(kBatchMaxThreads, K == 1 ? PGB_BATCH_MIN_BLOCK
   }
   __syncthreads();
   const int lane = threadIdx.x & (kWarp - 1);
-  const int wib = threadIdx.x >> 5;
-  // The arguments of the scene that the warp's ray belongs to, one copy per warp, rewritten
-  // when a ray of another scene comes (they are read where they are used: as local variables
-  // they and their spills took 140 bytes of stack in the 80-register kernel).
-  RenderArgs<float>& ra =
-      *reinterpret_cast<RenderArgs<float>*>(smem_raw + tab_bytes + (size_t)wib * kSceneArgsBytes);
   int current = -1;
-  BatchStage<K> cs(smem_raw + tab_bytes + (size_t)kSceneArgsBytes * (blockDim.x / kWarp), wib);
-
-  for (;;) {
-    unsigned long long rr = 0;
-    if (lane == 0) rr = atomicAdd(a.work, 1ull);
-    rr = __shfl_sync(kFull, rr, 0);
-    if ((int64_t)rr >= a.R) break;
-    const int64_t r = (int64_t)rr;
-    const int sid = a.ray_scene[r];
-    if ((unsigned)sid >= (unsigned)a.num_scenes) {  // not a scene of this batch: no work
-      if (lane == 0) a.ray_loss[r] = 0.f;
-      if (a.rgba_out != nullptr && lane < 4) a.rgba_out[4 * r + lane] = 0.f;
-      continue;
+  // Rays of one queue, each with its scene's arguments in place.
+  const auto for_rays = [&](unsigned long long* queue, auto&& body) {
+    for (;;) {
+      unsigned long long rr = 0;
+      if (lane == 0) rr = atomicAdd(queue, 1ull);
+      rr = __shfl_sync(kFull, rr, 0);
+      if ((int64_t)rr >= a.R) break;
+      const int64_t r = (int64_t)rr;
+      const int sid = a.ray_scene[r];
+      if ((unsigned)sid >= (unsigned)a.num_scenes) {  // not a scene of this batch: no work
+        if (lane == 0) a.ray_loss[r] = 0.f;
+        if (a.rgba_out != nullptr && lane < 4) a.rgba_out[4 * r + lane] = 0.f;
+        continue;
+      }
+      if (sid != current) {
+        __syncwarp();
+        if (lane == 0) scene_args<MODE>(a, sh.scenes[sid], ra);
+        __syncwarp();
+        current = sid;
+      }
+      body(sid, r);
     }
-    const pgb_scene& sc = sc_tab[sid];
-
-    if (sid != current) {
-      __syncwarp();
-      if (lane == 0) scene_args(a, sc, ra);
-      __syncwarp();
-      current = sid;
-    }
-    if (ra.g.quick)
-      batch_ray<Store, MODE, K, MERGE, kQuick>(a, sc, ra, r, cs, lane);
-    else
-      batch_ray_general<Store, MODE, K, MERGE>(a, sc, ra, r, cs, lane);
+  };
+  // 16 scenes of BF16, us: quick trilinear 1354 with the general form in a call beside it, 1411
+  // with it inline, 1280 with the others in a loop of their own; nearest 920 with a call or a
+  // second loop, 780 with both forms inline. All scenes at origin 0: trilinear 1529 (1923 by the
+  // call), nearest 860 (1126).
+  constexpr bool APART = MODE == PGB_TRILINEAR;
+  for_rays(a.work, [&](int sid, int64_t r) {
+    if (ra.g.quick == kSceneQuick)
+      batch_ray<Store, MODE, K, MERGE, kSceneQuick>(a, sh.scenes[sid], ra, r, sh.stage, lane);
+    else if (!APART)
+      batch_ray<Store, MODE, K, MERGE, kSceneGeneral>(a, sh.scenes[sid], ra, r, sh.stage, lane);
+  });
+  if constexpr (APART) {
+    bool others = false;
+    for (int i = lane; i < a.num_scenes; i += kWarp) others |= scene_arith<MODE>(sh.scenes[i]) != kSceneQuick;
+    if (__any_sync(kFull, others))
+      for_rays(a.work_others, [&](int sid, int64_t r) {
+        if (ra.g.quick == kSceneScaled)
+          batch_ray<Store, MODE, K, MERGE, kSceneScaled>(a, sh.scenes[sid], ra, r, sh.stage, lane);
+        else if (ra.g.quick == kSceneGeneral)
+          batch_ray_general<Store, MODE, K, MERGE>(a, sid, r, lane);
+      });
   }
 
   // the last block to finish resets the queue (ray_loss_sum_kernel, launched next, sums
@@ -401,7 +460,7 @@ __global__ void __launch_bounds__(kBatchMaxThreads, K == 1 ? PGB_BATCH_MIN_BLOCK
   if (threadIdx.x == 0) {
     __threadfence();
     if (atomicAdd(a.ticket, 1u) == gridDim.x - 1u) {
-      *a.work = 0ull;
+      *a.work = *a.work_others = 0ull;
       *a.ticket = 0u;
     }
   }
@@ -531,8 +590,7 @@ inline unsigned grid_for(int64_t n, int threads = 256) {
 template <typename Store, int MODE, int K, bool MERGE>
 int launch_batch_k(const BatchArgs& a, int threads, cudaStream_t s) {
   const int warps = threads / kWarp;
-  const size_t tab = (((size_t)a.num_scenes * sizeof(pgb_scene)) + 15) & ~(size_t)15;
-  const size_t smem = tab + (kSceneArgsBytes + (size_t)BatchStage<K>::kBytesPerWarp) * warps;
+  const size_t smem = BatchShared<K>::table_bytes(a.num_scenes) + (kSceneArgsBytes + (size_t)BatchStage<K>::kBytesPerWarp) * warps;
   auto kern = batch_train_kernel<Store, MODE, K, MERGE>;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -618,6 +676,7 @@ int pgb_batch_train(const pgb_scene* scenes, int32_t num_scenes, int32_t dtype, 
   a.loss_out = loss_out;
   a.work = reinterpret_cast<unsigned long long*>(workspace);
   a.ticket = reinterpret_cast<unsigned*>((char*)workspace + 8);
+  a.work_others = reinterpret_cast<unsigned long long*>((char*)workspace + 16);
   a.ray_loss = reinterpret_cast<float*>((char*)workspace + kRayLossOffset);
   const int merge = merge_updates ? 1 : 0;
   int st;

@@ -67,11 +67,13 @@ __device__ __forceinline__ bool use_quick(const GridP<Real>& g) {
 //    it is a multiple of an ulp of the smaller operand, beyond that it is at least half of
 //    |origin|), and pd within 2^+-40 keeps the rest normal.
 // Grids outside (a single cell along an axis has origin 0) take the general arithmetic.
+constexpr float kQuickMinOrigin = 9.5367431640625e-07f;  // 2^-20
+
 __host__ __device__ inline bool quick_grid(int X, int Y, int Z, float ox, float oy, float oz,
                                            float pd) {
   const auto fits = [](float o) {
     const float m = o < 0.f ? -o : o;
-    return m >= 9.5367431640625e-07f && m <= 1.0995116e12f;
+    return m >= kQuickMinOrigin && m <= 1.0995116e12f;
   };
   constexpr int kMaxDim = 1 << 21;
   return X <= kMaxDim && Y <= kMaxDim && Z <= kMaxDim &&
