@@ -188,10 +188,12 @@ __device__ __forceinline__ void scene_args(const BatchArgs& a, const pgb_scene& 
   ra.g.ox = scale * sc.origin[0]; ra.g.oy = scale * sc.origin[1]; ra.g.oz = scale * sc.origin[2];
   ra.g.pd = scale * sc.points_distance;
   ra.g.inv_pd = 1.0f / ra.g.pd;
+  set_box(ra.g);
   ra.g.clip = a.clip;
   ra.g.alpha_floor = 0.f;
   ra.S = sc.num_samples;
   ra.delta = sc.delta_step;
+  ra.inv_delta = 1.0f / sc.delta_step;
   ra.stratified = a.stratified;
   ra.grad = reinterpret_cast<float*>(sc.grad_cells);
 }
@@ -221,8 +223,11 @@ __device__ __forceinline__ void batch_ray(const BatchArgs& a, const pgb_scene& s
     if (a.rgba_out != nullptr && lane < 4) a.rgba_out[4 * r + lane] = __int_as_float(0x7fc00000);
     return;
   }
-  int first, end;
-  ray_span(ra, ray, first, end);
+  // Rays of up to four 32-sample chunks are not cut: it spares them a chunk at most, and delays the
+  // first (16 scenes of 128 samples: nearest 405 us cut, 392 whole; trilinear 811 and 804; at 300
+  // samples the cut gains 8 % and more).
+  int first = 0, end = ra.S;
+  if (ra.S > 4 * kWarp) ray_span(ra, ray, first, end);
   first -= first % (kWarp * K);  // chunks stay where they were: T is looked at after each
   const int nchunks = (end - first + kWarp * K - 1) / (kWarp * K);
   float v[K][4];

@@ -42,6 +42,7 @@ struct GridP {
   int clip;
   float alpha_floor;  // >0: clamped alpha below it reads as 0 (inference threshold)
   Real inv_pd;        // 1 / pd, rounded to nearest
+  Real box_lo[3], box_hi[3];  // the box of ray_span (set_box)
   int quick;          // the grid is in the range of the quick index arithmetic (quick_grid)
 };
 
@@ -131,7 +132,7 @@ struct RenderArgs {
   // sampling
   int64_t R;
   int S;
-  Real delta;
+  Real delta, inv_delta;
   int stratified;
   uint64_t strat_seed;
   int64_t first_ray;  // index of ray 0 in the stratification stream
@@ -297,14 +298,29 @@ __device__ __forceinline__ uint64_t cell_index(const GridP<Real>& g, int i, int 
 
 // The samples [first, end) of a ray outside of which every sample is out of bounds (value
 // 0, no gradient): the ray against the grid's box, grown by a hundredth of a cell and by
-// 2^-18 of the coordinates' magnitude (64 times what the rounding of a position can move
-// it), and two samples more at both ends (the jitter of stratified samples and the rounding
-// of the quotients). An axis whose bounds come out NaN restricts nothing, and neither does a
-// step that is not a positive normal number. `first` is a multiple of 32: the scans of a
-// slot then run over the samples that they would without the cut, with the same rounding.
-// Rays enter and leave the grid well inside their
-// [near, far] range, so this spares a quarter of the benchmark's samples: their chunks ran
-// the coordinate arithmetic and both scans for zeros.
+// 2^-18 of the coordinates' magnitude (64 times what the rounding of a position or of the
+// arithmetic here can move it), and two samples more at both ends (the jitter of stratified
+// samples and the rounding of the quotients). An axis whose bounds come out NaN restricts
+// nothing, and neither does a step that is not a positive normal number. `first` is a multiple of
+// 32: the scans of a slot then run over the samples that they would without the cut, with the
+// same rounding. Rays enter and leave the grid well inside their [near, far] range, so this
+// spares a quarter of the benchmark's samples: their chunks ran the coordinate arithmetic and
+// both scans for zeros. A ray of a few chunks may spare none, so the box and 1 / delta are
+// made once and the reciprocals are approximate ones.
+constexpr float kSpanSlack = 3.8147e-6f;  // 2^-18
+
+template <typename Real>
+__host__ __device__ inline void set_box(GridP<Real>& g) {
+  const Real org[3] = {g.ox, g.oy, g.oz}, dim[3] = {g.fX, g.fY, g.fZ};
+  const auto mag = [](Real x) { return x < Real(0) ? -x : x; };
+  for (int ax = 0; ax < 3; ++ax) {
+    const Real lo = org[ax] - Real(0.5) * g.pd, hi = org[ax] + dim[ax] * g.pd;
+    const Real grow = Real(0.01) * g.pd + Real(kSpanSlack) * (mag(lo) + mag(hi));
+    g.box_lo[ax] = lo - grow;
+    g.box_hi[ax] = hi + grow;
+  }
+}
+
 template <typename Real>
 __device__ __forceinline__ void ray_span(const RenderArgs<Real>& a, const Ray<Real>& ray, int& first,
                                          int& end) {
@@ -313,21 +329,20 @@ __device__ __forceinline__ void ray_span(const RenderArgs<Real>& a, const Ray<Re
   if constexpr (sizeof(Real) == 4) {
     if (!(a.delta >= 1e-30f) || !(a.g.pd > 0.f)) return;
     const float o[3] = {ray.ox, ray.oy, ray.oz}, d[3] = {ray.dx, ray.dy, ray.dz};
-    const float org[3] = {a.g.ox, a.g.oy, a.g.oz}, dim[3] = {a.g.fX, a.g.fY, a.g.fZ};
     float t0 = 0.f, t1 = __int_as_float(0x7f800000);
 #pragma unroll
     for (int ax = 0; ax < 3; ++ax) {
-      const float lo = org[ax] - 0.5f * a.g.pd, hi = org[ax] + dim[ax] * a.g.pd;
-      const float grow = 0.01f * a.g.pd + 3.8147e-6f * (fabsf(o[ax]) + fabsf(lo) + fabsf(hi));
-      const float inv = 1.0f / d[ax];
-      const float ta = (lo - grow - o[ax]) * inv, tb = (hi + grow - o[ax]) * inv;
+      const float slack = kSpanSlack * fabsf(o[ax]);
+      float inv;
+      asm("rcp.approx.f32 %0, %1;" : "=f"(inv) : "f"(d[ax]));
+      const float ta = (a.g.box_lo[ax] - o[ax] - slack) * inv, tb = (a.g.box_hi[ax] - o[ax] + slack) * inv;
       t0 = fmaxf(t0, fminf(ta, tb));  // fminf and fmaxf pass the other operand of a NaN
       t1 = fminf(t1, fmaxf(ta, tb));
     }
     // t of sample s lies in [delta * s, delta * (s + 1)]
-    const float inv = 1.0f / a.delta, most = (float)a.S;
-    first = (int)fminf(fmaxf(t0 * inv - 3.f, 0.f), most) & ~(kWarp - 1);
-    end = max(first, (int)fminf(fmaxf(t1 * inv + 3.f, 0.f), most));
+    const float most = (float)a.S;
+    first = (int)fminf(fmaxf(t0 * a.inv_delta - 3.f, 0.f), most) & ~(kWarp - 1);
+    end = max(first, (int)fminf(fmaxf(t1 * a.inv_delta + 3.f, 0.f), most));
   }
 }
 

@@ -36,6 +36,7 @@ GridP<Real> grid_params(const pgb_grid* g) {
   p.inv_pd = Real(1) / p.pd;
   p.quick = sizeof(Real) == 4 && quick_grid(p.X, p.Y, p.Z, (float)p.ox, (float)p.oy, (float)p.oz,
                                             (float)p.pd) ? 1 : 0;
+  set_box(p);
   p.clip = g->clip ? 1 : 0;
   p.alpha_floor = g->alpha_floor;
   return p;
@@ -83,6 +84,7 @@ RenderArgs<Real> render_args(const pgb_grid* g, const pgb_rays* r) {
   a.R = r->num_rays;
   a.S = r->num_samples;
   a.delta = (Real)r->delta_step;
+  a.inv_delta = Real(1) / a.delta;
   a.stratified = r->stratified ? 1 : 0;
   a.strat_seed = r->seed;
   a.first_ray = r->first_ray;
