@@ -88,16 +88,23 @@ def _render_forward(grid, origins, dirs, cfg, rgba=None):
     return rgba
 
 
+# (looked up once: a small launch waits for every microsecond of the host's)
+_transforms_active, _tracing_state = torch._C._are_functorch_transforms_active, torch._C._get_tracing_state
+_forward_ad = torch.autograd.forward_ad
+
+
 def _wants_autograd(*tensors):
     """Whether a call has to go through its autograd Function: a gradient may be asked for,
     a transform (vmap, forward-mode, functional tracing) is at work and decides itself, or the
     call is being traced (a trace records the Function as one operator, and a launch through a
     pointer not at all)."""
-    if torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0:
+    if _transforms_active() or _tracing_state() is not None or _forward_ad._current_level >= 0:
         return True
-    if torch.jit.is_tracing():
-        return True
-    return torch.is_grad_enabled() and any(t.requires_grad for t in tensors)
+    if torch.is_grad_enabled():
+        for t in tensors:
+            if t.requires_grad:
+                return True
+    return False
 
 
 class _RenderRays(torch.autograd.Function):
