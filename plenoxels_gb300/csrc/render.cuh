@@ -154,6 +154,7 @@ struct RenderArgs {
   int64_t clear_total16;
   uint32_t* clear_marks;
   int64_t clear_words;
+  int clear_first;  // a warp takes a round of the clear before each of its rays, not only after
   Real* loss_out;
   double* partials;  // fp64: block loss partials, and the block counter
   unsigned* counter;
@@ -1072,7 +1073,27 @@ render_kernel(const RenderArgs<Real> a) {
     return ray_of(__shfl_sync(kFull, taken, 0));
   };
 
+  // A round of the clear of the other gradient buffer: 32 mark words from a second counter of the
+  // block; false: none is left. On a stream of its own the clear took the SMs that the kernel's
+  // blocks were waiting for, and two event waits a step: nearest steps of 3500 rays x 140..320
+  // 46 -> 27 and 50 -> 40 us, 512^3 log-sum 378 -> 338 us. Warps take rounds when they have run out
+  // of rays, while the block's last ones run, or one before each ray as well (clear_first). Of the
+  // 8192-ray trilinear step's 95 us (256^3) the clear's 50 MB of zeros are about 15 and the
+  // marks 10.
+  const auto clear_round = [&]() -> bool {
+    const int64_t rounds = (a.clear_words + kWarp - 1) / kWarp;
+    unsigned taken = 0;
+    if (lane == 0) taken = atomicAdd(&s_cleared, 1u);
+    const int64_t round = (int64_t)blockIdx.x + (int64_t)gridDim.x * __shfl_sync(kFull, taken, 0);
+    if (round >= rounds) return false;
+    clear_marked_warp(a.clear_grad, a.clear_total16, kMarkCellsLog2, a.clear_marks, a.clear_words, round,
+                      rounds, lane);
+    return true;
+  };
+  bool to_clear = SUMS && a.clear_words > 0;
+
   for (int64_t r = QUEUE ? ray_of(threadIdx.x >> 5) : gw; r < a.R; r = next_ray(r)) {
+    if (SUMS && to_clear && a.clear_first) to_clear = clear_round();
     Ray<Real> ray;
     load_ray(a, r, ray, PHASE == kTrain);
     int first, end;
@@ -1286,23 +1307,7 @@ render_kernel(const RenderArgs<Real> a) {
   }
 
   if constexpr (SUMS) {
-    // The other buffer's units are cleared by the warps that have run out of rays, 32 mark words
-    // at a time from a second counter of the block, while the block's last rays run. On a stream
-    // of its own the clear took the SMs that the kernel's blocks were waiting for, and two event
-    // waits a step: nearest steps of 3500 rays x 140..320 46 -> 27 and 50 -> 40 us, 512^3 log-sum
-    // 378 -> 338 us. Of the 8192-ray trilinear step's 101 us (256^3) the clear's 50 MB of zeros
-    // still are 15 and the marks 10; clearing along with each ray instead took 104 us.
-    if (a.clear_words > 0) {
-      const int64_t rounds = (a.clear_words + kWarp - 1) / kWarp;
-      for (;;) {
-        unsigned taken = 0;
-        if (lane == 0) taken = atomicAdd(&s_cleared, 1u);
-        const int64_t round = (int64_t)blockIdx.x + (int64_t)gridDim.x * __shfl_sync(kFull, taken, 0);
-        if (round >= rounds) break;
-        clear_marked_warp(a.clear_grad, a.clear_total16, kMarkCellsLog2, a.clear_marks, a.clear_words, round,
-                          rounds, lane);
-      }
-    }
+    while (to_clear) to_clear = clear_round();
     // Warps add their bins up in shared memory and the block's last warp adds them to the
     // launch's, so that a block fences once, at its end (a fence at device scope also empties
     // the SM's L1: one per warp took the nearest step of 8192 rays from 44 to 66 us). The last
