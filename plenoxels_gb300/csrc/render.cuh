@@ -154,7 +154,7 @@ struct RenderArgs {
   int64_t clear_total16;
   uint32_t* clear_marks;
   int64_t clear_words;
-  int clear_first;  // a warp takes a round of the clear before each of its rays, not only after
+  int clear_early;  // some warps begin with the clear
   Real* loss_out;
   double* partials;  // fp64: block loss partials, and the block counter
   unsigned* counter;
@@ -1052,10 +1052,11 @@ render_kernel(const RenderArgs<Real> a) {
   __shared__ unsigned s_special[2];
   __shared__ unsigned s_taken;  // QUEUE: rays of this block that have a warp
   __shared__ unsigned s_cleared;  // SUMS: rounds of the clear that have a warp
+  const bool clear_early = SUMS && a.clear_early;
   if (QUEUE || PHASE == kTrain) {
     if (threadIdx.x == 0) {
       s_done = 0u;
-      s_taken = (unsigned)warps_per_block;
+      s_taken = clear_early ? 0u : (unsigned)warps_per_block;
       s_cleared = 0u;
     }
     if (SUMS && threadIdx.x < 2 * kWarp) s_bins[threadIdx.x >> 5][lane] = 0ull;
@@ -1077,9 +1078,9 @@ render_kernel(const RenderArgs<Real> a) {
   // block; false: none is left. On a stream of its own the clear took the SMs that the kernel's
   // blocks were waiting for, and two event waits a step: nearest steps of 3500 rays x 140..320
   // 46 -> 27 and 50 -> 40 us, 512^3 log-sum 378 -> 338 us. Warps take rounds when they have run out
-  // of rays, while the block's last ones run, or one before each ray as well (clear_first). Of the
-  // 8192-ray trilinear step's 95 us (256^3) the clear's 50 MB of zeros are about 15 and the
-  // marks 10.
+  // of rays, while the block's last ones run; in long launches some also take them before their
+  // first ray (clear_early). Of the 8192-ray trilinear step's 95 us (256^3) the clear's 50 MB of
+  // zeros are about 15 and the marks 10.
   const auto clear_round = [&]() -> bool {
     const int64_t rounds = (a.clear_words + kWarp - 1) / kWarp;
     unsigned taken = 0;
@@ -1090,10 +1091,16 @@ render_kernel(const RenderArgs<Real> a) {
                       rounds, lane);
     return true;
   };
-  bool to_clear = SUMS && a.clear_words > 0;
+  if (clear_early && (threadIdx.x & kWarp) != 0) {  // every other warp: three quarters of it
+    const unsigned early = (unsigned)(a.clear_words / (kWarp * (int64_t)gridDim.x) * 3 / 4);
+    const auto taken = [&]() -> unsigned {  // the same in every lane
+      return __shfl_sync(kFull, lane == 0 ? *(volatile unsigned*)&s_cleared : 0u, 0);
+    };
+    while (taken() < early && clear_round()) {
+    }
+  }
 
-  for (int64_t r = QUEUE ? ray_of(threadIdx.x >> 5) : gw; r < a.R; r = next_ray(r)) {
-    if (SUMS && to_clear && a.clear_first) to_clear = clear_round();
+  for (int64_t r = !QUEUE ? gw : clear_early ? next_ray(0) : ray_of(threadIdx.x >> 5); r < a.R; r = next_ray(r)) {
     Ray<Real> ray;
     load_ray(a, r, ray, PHASE == kTrain);
     int first, end;
@@ -1307,7 +1314,9 @@ render_kernel(const RenderArgs<Real> a) {
   }
 
   if constexpr (SUMS) {
-    while (to_clear) to_clear = clear_round();
+    if (a.clear_words > 0)
+      while (clear_round()) {
+      }
     // Warps add their bins up in shared memory and the block's last warp adds them to the
     // launch's, so that a block fences once, at its end (a fence at device scope also empties
     // the SM's L1: one per warp took the nearest step of 8192 rays from 44 to 66 us). The last

@@ -52,13 +52,13 @@ int launch_render_k(const RenderArgs<Real>& a, cudaStream_t s) {
   // / 676 us, half transparent 1913 / 1625 / 1630 / 1635 us.
   RenderArgs<Real> b = a;
   while (b.group_log2 < 3 && (a.R >> (b.group_log2 + 1)) >= 32 * blocks) ++b.group_log2;
-  // With two rays per warp or more the clear goes along with the first of them, while the
-  // gradient's atomics leave HBM idle, instead of behind the last. Only behind / along, us:
-  // half-transparent trilinear steps of 256^3, 8192 rays x 200 268 / 251, 20,000 rays 579 / 556;
-  // 400x400x293, 40,482 x 114 776 / 767; 512^3 log-sum of 65,536 rays 334 / 325; opaque 256^3, 8192
-  // rays x 256 90.8 / 91.0, 65,536 rays 471 / 462, 320^3 157 / 158; below two rays per warp,
-  // nearest 9000 rays 35 / 39.
-  b.clear_first = a.R >= 2 * blocks * kWarpsPerBlock ? 1 : 0;
+  // From five rays per warp on, every other warp begins with the clear, up to three quarters of
+  // it: the other warps' atomics leave HBM idle meanwhile, and hundreds of MB behind the last ray
+  // overlap with nothing. Only behind / three quarters early / all early, us: half-transparent
+  // trilinear steps, 256^3, 20,000 rays x 200 597 / 586 / 582, 400^3, 65,536 x 300 3280 / 3223 /
+  // 3211; 512^3 log-sum, 65,536 x 512 337 / 323 / 327; opaque 320^3, 40,000 x 256 103.6 / 104.1 /
+  // 106.6. With a round before every ray instead, inlined in the loop, every launch lost 2 %.
+  b.clear_early = a.clear_words > 0 && a.R >= 5 * blocks * kWarpsPerBlock ? 1 : 0;
   render_kernel<Real, Store, MODE, K, PHASE, LOGT, A><<<(unsigned)blocks, kThreads, kSmem, s>>>(b);
   return after_launch();
 }
