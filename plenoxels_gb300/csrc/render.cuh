@@ -1270,9 +1270,10 @@ render_kernel(const RenderArgs<Real> a) {
         Real fa = G * al, fb = Real(1) - al;
         if constexpr (MODE == PGB_NEAREST && K == 2 && sizeof(Real) == 4) {
           // The first step's a + b * a2 with a = G * al has two fused forms, an ulp apart. Rays
-          // of 128 samples and more without early stop were one long chunk, whose code fuses
-          // the other product; their bits stay as they were (the beta term's 1 / (1 - alpha +
-          // eps) turns an ulp of an opacity near 1 into 6e-4 of the next step's gradient).
+          // of more than 128 samples without early stop take the form that the code for 256-sample
+          // chunks has: a training run with the beta term, whose 1 / (1 - alpha + eps) turns an
+          // ulp of an opacity near 1 into 6e-4 of the next step's gradient, keeps its bits
+          // whether its chunks are picked, asked for at the same size, or of 256 samples.
           const Real a2 = __shfl_down_sync(kFull, fa, 1), b2 = __shfl_down_sync(kFull, fb, 1);
           const Real near = rfma(fb, a2, fa), far = rfma(G, al, rmul(fb, a2));
           if (lane < kWarp - 1) {

@@ -67,7 +67,7 @@ template <typename Real, typename Store, int MODE, int PHASE, bool LOGT, int A>
 int launch_render_mp(const RenderArgs<Real>& a, cudaStream_t s) {
   const bool early_stop = a.g.clip && !(PHASE == kTrain && a.beta_w != 0.0);
   RenderArgs<Real> b = a;
-  b.long_ray = MODE == PGB_NEAREST && !early_stop && a.chunk_samples <= 0 && a.S > 128;
+  b.long_ray = MODE == PGB_NEAREST && !early_stop && a.S > 128;
   const bool long_chunks = !early_stop && a.term_thr > 0.0f;
   switch (pick_slots(a.S, a.chunk_samples, MODE, long_chunks)) {
     case 1: return launch_render_k<Real, Store, MODE, 1, PHASE, LOGT, A>(b, s);
