@@ -284,6 +284,13 @@ __device__ __forceinline__ void sample_coords(const RenderArgs<Real>& a, const R
       nx = div_pd(x, a.g.pd, a.g.inv_pd);
       ny = div_pd(y, a.g.pd, a.g.inv_pd);
       nz = div_pd(z, a.g.pd, a.g.inv_pd);
+      if constexpr (A == kByGrid) {
+        // the views report the quotient also where it is not finite (the corrections make NaN of
+        // an infinity, which is as much out of bounds)
+        if (isinf(rdiv(x, a.g.pd))) nx = rdiv(x, a.g.pd);
+        if (isinf(rdiv(y, a.g.pd))) ny = rdiv(y, a.g.pd);
+        if (isinf(rdiv(z, a.g.pd))) nz = rdiv(z, a.g.pd);
+      }
     }
   } else {
     nx = rdiv(x, a.g.pd);
