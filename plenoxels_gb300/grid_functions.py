@@ -295,8 +295,15 @@ def convolve_grid_to_remove_noise(grid_cells, kernel_size=3, radius=1.0, thresho
     if not grid_cells.is_contiguous():
         raise ValueError("convolve_grid_to_remove_noise works in place on a contiguous grid")
     lib, dims = _lib.load(), _lib.dims3(grid_cells.shape)
-    scratch = torch.empty(max(16, lib.pgb_remove_noise_scratch_bytes(dims, int(repeats))),
-                          dtype=torch.uint8, device=grid_cells.device)
+    try:
+        scratch = torch.empty(max(16, lib.pgb_remove_noise_scratch_bytes(dims, int(repeats))),
+                              dtype=torch.uint8, device=grid_cells.device)
+    except torch.cuda.OutOfMemoryError:  # slower, with half the scratch
+        sums = torch.empty(grid_cells.shape[:3], dtype=torch.float32, device=grid_cells.device)
+        check(lib.pgb_remove_noise(ptr(grid_cells), dims, int(kernel_size), float(radius), float(threshold),
+                                   int(repeats), ptr(sums), stream_of(grid_cells)),
+              "convolve_grid_to_remove_noise")
+        return grid_cells
     check(lib.pgb_remove_noise_planes(ptr(grid_cells), dims, int(kernel_size), float(radius),
                                       float(threshold), int(repeats), ptr(scratch),
                                       stream_of(grid_cells)), "convolve_grid_to_remove_noise")
