@@ -20,7 +20,7 @@ from . import _lib
 from ._lib import check, ptr, require_cuda, stream_of
 from .grid_functions import grid_origin
 from .ray_sampling import _f32, generate_rays_batched
-from .render import _check_rays, _rays_desc, _render, _render_cfg
+from .render import _check_rays, _rays_desc, _render_cfg, _render_forward, _RenderRays, _wants_autograd
 
 PARAM_KEYS = ("device", "number_of_rays", "num_samples", "delta_step", "even_spread",
               "camera_ray", "points_distance", "gridsize")
@@ -107,6 +107,7 @@ def render_camera_images(grid, transforms, height, width, camera_angle_x, near, 
     lib, R = _lib.load(), H * W
     dirs = torch.empty(R, 3, dtype=torch.float32, device=dev)
     pixels = torch.empty(R, 4, dtype=torch.float32, device=dev)
+    plain = not _wants_autograd()  # no trace and no transform at work
     for c in range(C):
         T = _f32(transforms[c:c + 1], "render_camera_images")
         # the uniforms are pixel centres, inside the images by construction: no status word
@@ -114,5 +115,8 @@ def render_camera_images(grid, transforms, height, width, camera_angle_x, near, 
                                     ptr(pixels), None, stream_of(T)), "render_camera_images")
         origins = (T[0, :3, 3] + near * dirs).contiguous()
         _check_rays(g, origins, dirs)
-        _render(g, origins, dirs, cfg, out[c].view(R, 4))
+        if plain:
+            _render_forward(g, origins, dirs, cfg, out[c])
+        else:
+            out[c] = _RenderRays.apply(g, origins, dirs, cfg).reshape(H, W, 4)
     return out

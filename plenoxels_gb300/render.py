@@ -80,7 +80,7 @@ def _render_descs(grid, origins, dirs, cfg):
 
 
 def _render_forward(grid, origins, dirs, cfg, rgba=None):
-    """The forward launch; rgba: a contiguous [R,4] tensor to write to."""
+    """The forward launch; rgba: a contiguous tensor of R x 4 numbers to write to."""
     if rgba is None:
         rgba = torch.empty(origins.shape[0], 4, dtype=_lib.real_dtype(grid.dtype), device=grid.device)
     gdesc, rdesc = _render_descs(grid, origins, dirs, cfg)
@@ -150,15 +150,10 @@ def render_rays(grid, origins, dirs, delta_step, num_samples, points_distance, g
         grid_min = grid_origin(grid.shape, points_distance, _lib.real_dtype(grid.dtype))
     cfg = _render_cfg(grid_min, points_distance, mode, delta_step, num_samples, clip, stratified, seed,
                       term_threshold, background, transmittance, chunk_samples)
-    return _render(grid.contiguous(), origins.contiguous(), dirs.contiguous(), cfg)
-
-
-def _render(grid, origins, dirs, cfg, rgba=None):
-    """The checked rays' pixels; rgba: a contiguous [R,4] tensor for them (no gradient then)."""
+    grid, origins, dirs = grid.contiguous(), origins.contiguous(), dirs.contiguous()
     if not _wants_autograd(grid, origins, dirs):
-        return _render_forward(grid, origins, dirs, cfg, rgba)
-    out = _RenderRays.apply(grid, origins, dirs, cfg)
-    return out if rgba is None else rgba.copy_(out)
+        return _render_forward(grid, origins, dirs, cfg)
+    return _RenderRays.apply(grid, origins, dirs, cfg)
 
 
 def render_sample_indices(grid, origins, dirs, delta_step, num_samples, points_distance,
