@@ -291,7 +291,8 @@ class FusedTrainStep:
             if zeroing != "marked":
                 self._side = torch.cuda.Stream(device=dev)
             self._zeroed = [None, None]  # buffer b is zero and free: an event (fill), True (marked)
-        # whether a CUDA graph holds steps of two marked buffers: what a step leaves zeroed is then
+        self._pair = overlap_zero and zeroing == "marked"  # two buffers, cleared by the kernels
+        # whether a CUDA graph holds steps of such a pair: what a step leaves zeroed is then
         # no longer what the next one finds (replays come in between), so each clears its own
         self._captured = False
         if zeroing not in ("fill", "marked"):
@@ -331,7 +332,7 @@ class FusedTrainStep:
             self._fill(0, stream_of(self.grid))
             self._buf = 0
             return self.grad
-        if self._side is None:
+        if self._pair:
             b = self._cur
             if self._captured or not self._zeroed[b]:
                 self._fill(b, stream_of(self.grid))
@@ -382,8 +383,7 @@ class FusedTrainStep:
         lib = _lib.load()
         losses = self._loss_target(loss_out)
         self.launches += 1
-        marked_pair = self._side is None and len(self._grads) == 2
-        if marked_pair and torch.cuda.is_current_stream_capturing():
+        if self._pair and torch.cuda.is_current_stream_capturing():
             self._captured = True
         grad = self._gradient_for_step(zero_grad)
         if self._marks is not None:
@@ -395,7 +395,7 @@ class FusedTrainStep:
             main = torch.cuda.current_stream(self.grid.device)
             ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
             ev[0].record(main)
-        if zero_grad and marked_pair and not self._captured:
+        if self._pair and zero_grad and not self._captured:
             o = 1 - self._buf
             terms = _lib.PgbLossTerms(self.loss_weight, self.beta, self.beta_eps)
             check(lib.pgb_render_train_clear(gdesc, rdesc, ptr(target), terms, ptr(rgba_out), ptr(grad),
