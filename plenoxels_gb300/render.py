@@ -245,13 +245,14 @@ class FusedTrainStep:
 
     overlap_zero=True keeps two gradient buffers and zeroes the next step's buffer while the
     current step's kernel runs (the 256 MiB fill of a 256^3 grid no longer sits on the
-    critical path): on a side stream, or with zeroing="marked" in the kernel itself. A step's gradient then stays valid until the
-    next step is launched; the buffer alternates, and ``grid.grad``/``self.grad`` follow.
+    critical path): on a side stream, or with zeroing="marked" in the kernel itself. A step's
+    gradient then stays valid until the next step is launched; the buffer alternates, and
+    ``grid.grad``/``self.grad`` follow.
 
     zeroing="marked" re-zeroes a gradient buffer by clearing only the 4-cell units its
     last step wrote (the kernel marks them in a bitmap of the buffer, pgb_clear_marked)
-    instead of writing the whole buffer (grids of up to MARKED_CELLS cells are cleared whole). Every step still starts from an all-zero dense
-    gradient, provided the caller only reads the gradient buffers (an optimizer that
+    instead of writing the whole buffer (grids of up to MARKED_CELLS cells are cleared whole).
+    Every step still starts from an all-zero dense gradient, provided the caller only reads the gradient buffers (an optimizer that
     reads grid.grad, or zeroes it) and does not add into them; an in-place all-reduce of
     the gradient over ranks adds into them.
     """
