@@ -89,7 +89,7 @@ def _render_forward(grid, origins, dirs, cfg, rgba=None):
 
 
 # (looked up once: a small launch waits for every microsecond of the host's)
-_transforms_active, _tracing_state = torch._C._are_functorch_transforms_active, torch._C._get_tracing_state
+_transforms_active, _is_tracing = torch._C._are_functorch_transforms_active, torch._C._is_tracing
 _forward_ad = torch.autograd.forward_ad
 
 
@@ -98,7 +98,7 @@ def _wants_autograd(*tensors):
     a transform (vmap, forward-mode, functional tracing) is at work and decides itself, or the
     call is being traced (a trace records the Function as one operator, and a launch through a
     pointer not at all)."""
-    if _transforms_active() or _tracing_state() is not None or _forward_ad._current_level >= 0:
+    if _transforms_active() or _is_tracing() or _forward_ad._current_level >= 0:
         return True
     if torch.is_grad_enabled():
         for t in tensors:
