@@ -159,8 +159,8 @@ int pgb_render_train_terms(const pgb_grid* grid, const pgb_rays* rays, const voi
                            void* losses_out, void* workspace, pgb_stream_t stream);
 /* pgb_render_train_terms that also zeroes the marked units of another gradient buffer of the
  * grid's dims and clears its marks (pgb_clear_marked; without marks it zeroes the whole buffer),
- * with the warps that have no ray left: for callers that keep two buffers and clear the next
- * step's during this one. */
+ * with warps that have no ray left, in long launches also with some before their first ray: for
+ * callers that keep two buffers and clear the next step's during this one. */
 int pgb_render_train_clear(const pgb_grid* grid, const pgb_rays* rays, const void* target,
                            const pgb_loss_terms* terms, void* rgba_out, void* grad_cells,
                            void* losses_out, void* workspace, void* clear_grad_cells,

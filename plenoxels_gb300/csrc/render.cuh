@@ -67,7 +67,8 @@ __device__ __forceinline__ bool use_quick(const GridP<Real>& g) {
 //    the difference p - origin is 0 or at least 2^-45 in magnitude (below a factor of two
 //    it is a multiple of an ulp of the smaller operand, beyond that it is at least half of
 //    |origin|), and pd within 2^+-40 keeps the rest normal.
-// Grids outside (a single cell along an axis has origin 0) take the general arithmetic.
+// Grids outside (an axis of one or two cells has origin 0, and a caller may give it) take the
+// general arithmetic.
 constexpr float kQuickMinOrigin = 9.5367431640625e-07f;  // 2^-20
 
 __host__ __device__ inline bool quick_grid(int X, int Y, int Z, float ox, float oy, float oz,
